@@ -4,7 +4,7 @@
 // preconditioned residual norm in KSPConvergedDefault, breakdown when
 // (v, rp) = 0 or rho = 0, and the t = 0 exit (x += alpha p) of the omega
 // step.  Every scalar lives in a device control block updated by the last
-// CTA of a deterministic reduction (fixed grid, fixed order), so iterations
+// CTA of a deterministic reduction (grid and order fixed by n), so iterations
 // can be enqueued in CUDA-graph chunks without host round trips; once the
 // solve has ended every kernel of a later iteration returns at once.
 //
@@ -59,6 +59,79 @@ __global__ void bcgs_setup(BcgsState *st, int maxit, double rtol, double atol, d
   st->counter = 0u;
 }
 
+// Reductions.  A kernel's CTAs leave one partial sum each; the last CTA to
+// arrive adds them with all its threads (a fixed tree), and a small vector gets a
+// small grid.  With 296 CTAs always and one thread adding 296 partials, alpha,
+// omega and xr took 8.7, 24.3 and 12.6 us on 6,912 dofs and 14.5, 29.6 and 23.9 on
+// 1.1 M; now 4.2, 5.0, 5.8 and 9.4, 11.4, 15.5 (1.1 M: bound by the vectors' 9 MB
+// each from L2).  Inner products are carried as unevaluated pairs hi + lo
+// (products split exactly by FMA, Knuth's two-sum; Ogita, Rump and Oishi, 2005):
+// BiCGStab's (r, rp) and (v, rp) fall many orders below the sum of their terms'
+// magnitudes, and a plain sum can then cancel to exactly 0.0, which the
+// breakdown rule takes for an orthogonal vector.
+struct Pair {
+  double hi, lo;
+};
+
+__device__ __forceinline__ Pair pair_add(const Pair &a, const Pair &b)
+{
+  const double s = a.hi + b.hi, t = s - a.hi;
+  return {s, (a.lo + b.lo) + ((a.hi - (s - t)) + (b.hi - t))};
+}
+
+__device__ __forceinline__ void pair_fma(Pair &acc, double x, double y)
+{
+  const double p = x * y;
+  acc = pair_add(acc, {p, fma(x, y, -p)});
+}
+
+// sum over the CTA, valid in every thread; sh: RED_THREADS / 32 entries
+__device__ __forceinline__ Pair block_sum_pair(Pair v, Pair *sh)
+{
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1)
+    v = pair_add(v, {__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
+  __syncthreads();
+  if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = v;
+  __syncthreads();
+  v = sh[0];
+#pragma unroll
+  for (int k = 1; k < RED_THREADS / 32; k++) v = pair_add(v, sh[k]);
+  return v;
+}
+
+// CTAs of a reduction over n entries: four entries per thread, at most RED_BLOCKS
+inline int red_grid(int64_t n)
+{
+  const int64_t g = (n + 4 * RED_THREADS - 1) / (4 * RED_THREADS);
+  return (int)(g < 1 ? 1 : g > RED_BLOCKS ? RED_BLOCKS : g);
+}
+
+// The CTA's K sums to memory; true in the last CTA to arrive, whose threads
+// then all hold the K totals in v.  partial: 2 * K * gridDim.x doubles.
+template <int K>
+__device__ __forceinline__ bool reduce_all(Pair (&v)[K], double *__restrict__ partial, unsigned int *counter)
+{
+  __shared__ Pair sh[RED_THREADS / 32];
+  Pair *const mine = reinterpret_cast<Pair *>(partial);
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    const Pair t = block_sum_pair(v[q], sh);
+    if (threadIdx.x == 0) mine[q * gridDim.x + blockIdx.x] = t;
+  }
+  if (!last_block(counter, gridDim.x)) return false;
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    Pair t{0.0, 0.0};
+    for (unsigned int k = threadIdx.x; k < gridDim.x; k += RED_THREADS) {
+      const double2 p = __ldcg(reinterpret_cast<const double2 *>(partial) + q * gridDim.x + k);
+      t = pair_add(t, {p.x, p.y});
+    }
+    v[q] = block_sum_pair(t, sh);
+  }
+  return true;
+}
+
 // Start: r holds M^-1 b.  rp = r, p = v = 0, dp = ||r||, rho = (r, rp),
 // convergence test at iteration 0.
 template <typename VT>
@@ -67,32 +140,26 @@ bcgs_init(int64_t n, const VT *__restrict__ r, VT *__restrict__ rp, VT *__restri
           BcgsState *st, double *__restrict__ partial)
 {
   if (st->skip) return;
-  __shared__ double sh[RED_THREADS / 32];
-  double s = 0.0;
+  Pair s[1] = {{0.0, 0.0}};
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
     const VT x = r[i];
     rp[i] = x;
     p[i] = VT(0);
     v[i] = VT(0);
-    s = fma((double)x, (double)x, s);
+    pair_fma(s[0], (double)x, (double)x);
   }
-  s = block_sum<RED_THREADS>(s, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
-  if (last_block(&st->counter, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) t += __ldcg(partial + k);
-      const double dp = sqrt(t);
-      st->dp = dp;
-      st->its = 0;
-      const int reason = bcgs_converged(st, 0, dp);
-      st->reason = reason;
-      st->active = (reason == 0 && st->maxit > 0) ? 1 : 0;
-      // first iteration: rho = (r, rp), beta = (rho / 1) (1 / 1)
-      st->rho = t;
-      st->rhoold = 1.0; st->alpha = 1.0; st->omegaold = 1.0;
-      st->beta = (st->rho / st->rhoold) * (st->alpha / st->omegaold);
-    }
+  if (reduce_all(s, partial, &st->counter) && threadIdx.x == 0) {
+    const double t = s[0].hi + s[0].lo;
+    const double dp = sqrt(t);
+    st->dp = dp;
+    st->its = 0;
+    const int reason = bcgs_converged(st, 0, dp);
+    st->reason = reason;
+    st->active = (reason == 0 && st->maxit > 0) ? 1 : 0;
+    // first iteration: rho = (r, rp), beta = (rho / 1) (1 / 1)
+    st->rho = t;
+    st->rhoold = 1.0; st->alpha = 1.0; st->omegaold = 1.0;
+    st->beta = (st->rho / st->rhoold) * (st->alpha / st->omegaold);
   }
 }
 
@@ -112,23 +179,18 @@ __global__ void __launch_bounds__(RED_THREADS)
 bcgs_alpha(int64_t n, const VT *__restrict__ v, const VT *__restrict__ rp, BcgsState *st, double *__restrict__ partial)
 {
   if (!st->active) return;
-  __shared__ double sh[RED_THREADS / 32];
-  double s = 0.0;
+  Pair s[1] = {{0.0, 0.0}};
+#pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS)
-    s = fma((double)v[i], (double)rp[i], s);
-  s = block_sum<RED_THREADS>(s, sh);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
-  if (last_block(&st->counter, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      double d1 = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) d1 += __ldcg(partial + k);
-      if (isnan(d1) || isinf(d1)) {
-        st->reason = -9; st->active = 0;      // KSP_DIVERGED_NANORINF
-      } else if (d1 == 0.0) {
-        st->reason = -5; st->active = 0;      // KSP_DIVERGED_BREAKDOWN
-      } else {
-        st->alpha = st->rho / d1;
-      }
+    pair_fma(s[0], (double)v[i], (double)rp[i]);
+  if (reduce_all(s, partial, &st->counter) && threadIdx.x == 0) {
+    const double d1 = s[0].hi + s[0].lo;
+    if (isnan(d1) || isinf(d1)) {
+      st->reason = -9; st->active = 0;      // KSP_DIVERGED_NANORINF
+    } else if (d1 == 0.0) {
+      st->reason = -5; st->active = 0;      // KSP_DIVERGED_BREAKDOWN
+    } else {
+      st->alpha = st->rho / d1;
     }
   }
 }
@@ -150,40 +212,25 @@ __global__ void __launch_bounds__(RED_THREADS)
 bcgs_omega(int64_t n, const VT *__restrict__ s, const VT *__restrict__ t, BcgsState *st, double *__restrict__ partial)
 {
   if (!st->active) return;
-  __shared__ double sh[RED_THREADS / 32];
-  double a = 0.0, b = 0.0, c = 0.0;
+  Pair d[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
     const double si = (double)s[i], ti = (double)t[i];
-    a = fma(si, ti, a);
-    b = fma(ti, ti, b);
-    c = fma(si, si, c);
+    pair_fma(d[0], si, ti);
+    pair_fma(d[1], ti, ti);
+    pair_fma(d[2], si, si);
   }
-  a = block_sum<RED_THREADS>(a, sh);
-  b = block_sum<RED_THREADS>(b, sh);
-  c = block_sum<RED_THREADS>(c, sh);
-  if (threadIdx.x == 0) {
-    partial[3 * blockIdx.x] = a;
-    partial[3 * blockIdx.x + 1] = b;
-    partial[3 * blockIdx.x + 2] = c;
-  }
-  if (last_block(&st->counter, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      double d1 = 0.0, d2 = 0.0, d3 = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) {
-        d1 += __ldcg(partial + 3 * k);
-        d2 += __ldcg(partial + 3 * k + 1);
-        d3 += __ldcg(partial + 3 * k + 2);
-      }
-      if (d2 == 0.0) {
-        if (d3 != 0.0) {
-          st->reason = -5; st->active = 0;    // singular preconditioned operator
-        } else {
-          st->tzero = 1;
-          st->omega = 0.0;
-        }
+  if (reduce_all(d, partial, &st->counter) && threadIdx.x == 0) {
+    const double d1 = d[0].hi + d[0].lo, d2 = d[1].hi + d[1].lo, d3 = d[2].hi + d[2].lo;
+    if (d2 == 0.0) {
+      if (d3 != 0.0) {
+        st->reason = -5; st->active = 0;    // singular preconditioned operator
       } else {
-        st->omega = d1 / d2;
+        st->tzero = 1;
+        st->omega = 0.0;
       }
+    } else {
+      st->omega = d1 / d2;
     }
   }
 }
@@ -196,10 +243,10 @@ bcgs_xr(int64_t n, double *__restrict__ x, const VT *__restrict__ p, const VT *_
         VT *__restrict__ r, const VT *__restrict__ rp, BcgsState *st, double *__restrict__ partial)
 {
   if (!st->active) return;
-  __shared__ double sh[RED_THREADS / 32];
   const double alpha = st->alpha, omega = st->omega;
   const bool tz = st->tzero != 0;
-  double a = 0.0, b = 0.0;
+  Pair d[2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll 2
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
     if (tz) {
       x[i] += alpha * (double)p[i];
@@ -208,42 +255,29 @@ bcgs_xr(int64_t n, double *__restrict__ x, const VT *__restrict__ p, const VT *_
       const VT ri = (VT)(-omega * (double)t[i] + (double)s[i]);
       r[i] = ri;
       const double rd = (double)ri;
-      a = fma(rd, rd, a);
-      b = fma(rd, (double)rp[i], b);
+      pair_fma(d[0], rd, rd);
+      pair_fma(d[1], rd, (double)rp[i]);
     }
   }
-  a = block_sum<RED_THREADS>(a, sh);
-  b = block_sum<RED_THREADS>(b, sh);
-  if (threadIdx.x == 0) {
-    partial[2 * blockIdx.x] = a;
-    partial[2 * blockIdx.x + 1] = b;
-  }
-  if (last_block(&st->counter, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      st->its = st->its + 1;
-      if (tz) {
-        st->dp = 0.0;
-        st->reason = 2;                       // KSP_CONVERGED_RTOL
-        st->active = 0;
-      } else {
-        double rr = 0.0, rrp = 0.0;
-        for (unsigned int k = 0; k < gridDim.x; k++) {
-          rr += __ldcg(partial + 2 * k);
-          rrp += __ldcg(partial + 2 * k + 1);
-        }
-        const double dp = sqrt(rr);
-        st->dp = dp;
-        const double rho = st->rho;
-        st->rhoold = rho;
-        st->omegaold = omega;
-        int reason = bcgs_converged(st, st->its, dp);
-        if (reason == 0 && rho == 0.0) reason = -5;
-        if (reason == 0 && st->its >= st->maxit) reason = -3;   // KSP_DIVERGED_ITS
-        st->reason = reason;
-        st->active = (reason == 0) ? 1 : 0;
-        st->rho = rrp;
-        st->beta = (st->rho / st->rhoold) * (st->alpha / st->omegaold);
-      }
+  if (reduce_all(d, partial, &st->counter) && threadIdx.x == 0) {
+    st->its = st->its + 1;
+    if (tz) {
+      st->dp = 0.0;
+      st->reason = 2;                       // KSP_CONVERGED_RTOL
+      st->active = 0;
+    } else {
+      const double dp = sqrt(d[0].hi + d[0].lo);
+      st->dp = dp;
+      const double rho = st->rho;
+      st->rhoold = rho;
+      st->omegaold = omega;
+      int reason = bcgs_converged(st, st->its, dp);
+      if (reason == 0 && rho == 0.0) reason = -5;
+      if (reason == 0 && st->its >= st->maxit) reason = -3;   // KSP_DIVERGED_ITS
+      st->reason = reason;
+      st->active = (reason == 0) ? 1 : 0;
+      st->rho = d[1].hi + d[1].lo;
+      st->beta = (st->rho / st->rhoold) * (st->alpha / st->omegaold);
     }
   }
 }
