@@ -85,6 +85,27 @@ __device__ __forceinline__ void pair_fma(Pair &acc, double x, double y)
   acc = pair_add(acc, {p, fma(x, y, -p)});
 }
 
+// CTAs of a reduction over n entries: four entries per thread, at most RED_BLOCKS
+inline int red_grid(int64_t n)
+{
+  const int64_t g = (n + 4 * RED_THREADS - 1) / (4 * RED_THREADS);
+  return (int)(g < 1 ? 1 : g > RED_BLOCKS ? RED_BLOCKS : g);
+}
+
+// FP32 vectors (the inner solves of the mixed-precision path) have products that
+// are exact in 64 bits and a tolerance of a digit or two: plain sums, and always in
+// the same order (RED_BLOCKS CTAs, their partials one after another), because the
+// outer solve carries the last bit of alpha and omega on into the pressure level
+// that it ends at.  The partials are loaded by all threads and added from shared memory.
+template <typename VT> struct SumOf { using type = Pair; };
+template <> struct SumOf<float> { using type = double; };
+template <typename VT> using Sum = typename SumOf<VT>::type;
+template <typename VT> inline int bcgs_grid(int64_t n) { return sizeof(VT) == 4 ? RED_BLOCKS : red_grid(n); }
+__device__ __forceinline__ void sum_fma(Pair &acc, double x, double y) { pair_fma(acc, x, y); }
+__device__ __forceinline__ void sum_fma(double &acc, double x, double y) { acc = fma(x, y, acc); }
+__device__ __forceinline__ double sum_value(const Pair &v) { return v.hi + v.lo; }
+__device__ __forceinline__ double sum_value(double v) { return v; }
+
 // sum over the CTA, valid in every thread; sh: RED_THREADS / 32 entries
 __device__ __forceinline__ Pair block_sum_pair(Pair v, Pair *sh)
 {
@@ -98,13 +119,6 @@ __device__ __forceinline__ Pair block_sum_pair(Pair v, Pair *sh)
 #pragma unroll
   for (int k = 1; k < RED_THREADS / 32; k++) v = pair_add(v, sh[k]);
   return v;
-}
-
-// CTAs of a reduction over n entries: four entries per thread, at most RED_BLOCKS
-inline int red_grid(int64_t n)
-{
-  const int64_t g = (n + 4 * RED_THREADS - 1) / (4 * RED_THREADS);
-  return (int)(g < 1 ? 1 : g > RED_BLOCKS ? RED_BLOCKS : g);
 }
 
 // The CTA's K sums to memory; true in the last CTA to arrive, whose threads
@@ -132,6 +146,25 @@ __device__ __forceinline__ bool reduce_all(Pair (&v)[K], double *__restrict__ pa
   return true;
 }
 
+template <int K>
+__device__ __forceinline__ bool reduce_all(double (&v)[K], double *__restrict__ partial, unsigned int *counter)
+{
+  __shared__ double sh[RED_THREADS / 32], all[K * RED_BLOCKS], total[K];
+#pragma unroll
+  for (int q = 0; q < K; q++) {
+    const double t = block_sum<RED_THREADS>(v[q], sh);
+    if (threadIdx.x == 0) partial[q * gridDim.x + blockIdx.x] = t;
+  }
+  if (!last_block(counter, gridDim.x)) return false;
+  for (unsigned int k = threadIdx.x; k < K * gridDim.x; k += RED_THREADS) all[k] = __ldcg(partial + k);
+  __syncthreads();
+  if (threadIdx.x < K) total[threadIdx.x] = sum_in_order(all + threadIdx.x * gridDim.x, gridDim.x);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < K; q++) v[q] = total[q];
+  return true;
+}
+
 // Start: r holds M^-1 b.  rp = r, p = v = 0, dp = ||r||, rho = (r, rp),
 // convergence test at iteration 0.
 template <typename VT>
@@ -140,16 +173,16 @@ bcgs_init(int64_t n, const VT *__restrict__ r, VT *__restrict__ rp, VT *__restri
           BcgsState *st, double *__restrict__ partial)
 {
   if (st->skip) return;
-  Pair s[1] = {{0.0, 0.0}};
+  Sum<VT> s[1] = {};
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
     const VT x = r[i];
     rp[i] = x;
     p[i] = VT(0);
     v[i] = VT(0);
-    pair_fma(s[0], (double)x, (double)x);
+    sum_fma(s[0], (double)x, (double)x);
   }
   if (reduce_all(s, partial, &st->counter) && threadIdx.x == 0) {
-    const double t = s[0].hi + s[0].lo;
+    const double t = sum_value(s[0]);
     const double dp = sqrt(t);
     st->dp = dp;
     st->its = 0;
@@ -179,12 +212,12 @@ __global__ void __launch_bounds__(RED_THREADS)
 bcgs_alpha(int64_t n, const VT *__restrict__ v, const VT *__restrict__ rp, BcgsState *st, double *__restrict__ partial)
 {
   if (!st->active) return;
-  Pair s[1] = {{0.0, 0.0}};
+  Sum<VT> s[1] = {};
 #pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS)
-    pair_fma(s[0], (double)v[i], (double)rp[i]);
+    sum_fma(s[0], (double)v[i], (double)rp[i]);
   if (reduce_all(s, partial, &st->counter) && threadIdx.x == 0) {
-    const double d1 = s[0].hi + s[0].lo;
+    const double d1 = sum_value(s[0]);
     if (isnan(d1) || isinf(d1)) {
       st->reason = -9; st->active = 0;      // KSP_DIVERGED_NANORINF
     } else if (d1 == 0.0) {
@@ -212,16 +245,16 @@ __global__ void __launch_bounds__(RED_THREADS)
 bcgs_omega(int64_t n, const VT *__restrict__ s, const VT *__restrict__ t, BcgsState *st, double *__restrict__ partial)
 {
   if (!st->active) return;
-  Pair d[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+  Sum<VT> d[3] = {};
 #pragma unroll 4
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
     const double si = (double)s[i], ti = (double)t[i];
-    pair_fma(d[0], si, ti);
-    pair_fma(d[1], ti, ti);
-    pair_fma(d[2], si, si);
+    sum_fma(d[0], si, ti);
+    sum_fma(d[1], ti, ti);
+    sum_fma(d[2], si, si);
   }
   if (reduce_all(d, partial, &st->counter) && threadIdx.x == 0) {
-    const double d1 = d[0].hi + d[0].lo, d2 = d[1].hi + d[1].lo, d3 = d[2].hi + d[2].lo;
+    const double d1 = sum_value(d[0]), d2 = sum_value(d[1]), d3 = sum_value(d[2]);
     if (d2 == 0.0) {
       if (d3 != 0.0) {
         st->reason = -5; st->active = 0;    // singular preconditioned operator
@@ -245,7 +278,7 @@ bcgs_xr(int64_t n, double *__restrict__ x, const VT *__restrict__ p, const VT *_
   if (!st->active) return;
   const double alpha = st->alpha, omega = st->omega;
   const bool tz = st->tzero != 0;
-  Pair d[2] = {{0.0, 0.0}, {0.0, 0.0}};
+  Sum<VT> d[2] = {};
 #pragma unroll 2
   for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
     if (tz) {
@@ -255,8 +288,8 @@ bcgs_xr(int64_t n, double *__restrict__ x, const VT *__restrict__ p, const VT *_
       const VT ri = (VT)(-omega * (double)t[i] + (double)s[i]);
       r[i] = ri;
       const double rd = (double)ri;
-      pair_fma(d[0], rd, rd);
-      pair_fma(d[1], rd, (double)rp[i]);
+      sum_fma(d[0], rd, rd);
+      sum_fma(d[1], rd, (double)rp[i]);
     }
   }
   if (reduce_all(d, partial, &st->counter) && threadIdx.x == 0) {
@@ -266,7 +299,7 @@ bcgs_xr(int64_t n, double *__restrict__ x, const VT *__restrict__ p, const VT *_
       st->reason = 2;                       // KSP_CONVERGED_RTOL
       st->active = 0;
     } else {
-      const double dp = sqrt(d[0].hi + d[0].lo);
+      const double dp = sqrt(sum_value(d[0]));
       st->dp = dp;
       const double rho = st->rho;
       st->rhoold = rho;
@@ -276,7 +309,7 @@ bcgs_xr(int64_t n, double *__restrict__ x, const VT *__restrict__ p, const VT *_
       if (reason == 0 && st->its >= st->maxit) reason = -3;   // KSP_DIVERGED_ITS
       st->reason = reason;
       st->active = (reason == 0) ? 1 : 0;
-      st->rho = d[1].hi + d[1].lo;
+      st->rho = sum_value(d[1]);
       st->beta = (st->rho / st->rhoold) * (st->alpha / st->omegaold);
     }
   }

@@ -881,7 +881,7 @@ static int bcgs(cfdgpu_handle *h, const double *b, double *x, int *its_out, int 
   LAUNCHED(h);
   CK(cudaMemsetAsync(x, 0, sizeof(double) * n, h->stream));
   if ((rc = pc_apply_vec(h, b, h->bR))) return rc;
-  bcgs_init<double><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, h->bR, h->bRP, h->bP, h->bV, st, h->red_partial2);
+  bcgs_init<double><<<bcgs_grid<double>(n), RED_THREADS, 0, h->stream>>>(n, h->bR, h->bRP, h->bP, h->bV, st, h->red_partial2);
   LAUNCHED(h);
   if ((rc = check_launch(h, "bcgs_init"))) return rc;
   const int vgrid = grid_for(n);
@@ -893,13 +893,13 @@ static int bcgs(cfdgpu_handle *h, const double *b, double *x, int *its_out, int 
     prof_end(h, pi);
     if ((r = spmv_pc(h, 0, h->bP, nullptr, h->bV, nullptr, 0, nullptr, act))) return r;
     pi = prof_begin(h, CFDGPU_KIND_BCGS, 5.0 * V);
-    bcgs_alpha<double><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, h->bV, h->bRP, st, h->red_partial2);
+    bcgs_alpha<double><<<bcgs_grid<double>(n), RED_THREADS, 0, h->stream>>>(n, h->bV, h->bRP, st, h->red_partial2);
     bcgs_s<double><<<vgrid, 256, 0, h->stream>>>(n, h->bR, h->bV, h->bS, st);
     prof_end(h, pi);
     if ((r = spmv_pc(h, 0, h->bS, nullptr, h->bT, nullptr, 0, nullptr, act))) return r;
     pi = prof_begin(h, CFDGPU_KIND_BCGS, 10.0 * V);
-    bcgs_omega<double><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, h->bS, h->bT, st, h->red_partial2);
-    bcgs_xr<double><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, x, h->bP, h->bS, h->bT, h->bR, h->bRP, st,
+    bcgs_omega<double><<<bcgs_grid<double>(n), RED_THREADS, 0, h->stream>>>(n, h->bS, h->bT, st, h->red_partial2);
+    bcgs_xr<double><<<bcgs_grid<double>(n), RED_THREADS, 0, h->stream>>>(n, x, h->bP, h->bS, h->bT, h->bR, h->bRP, st,
                                                               h->red_partial2);
     prof_end(h, pi);
     h->launches += 5;
@@ -1003,17 +1003,17 @@ static int inner_bcgs32(cfdgpu_handle *h, const double *vj, const double *sigma_
   h->launches += 2;
   CK(cudaMemsetAsync(z, 0, sizeof(double) * n, h->stream));
   if ((rc = pc32_apply_vec(h, h->b32, h->iR, ost, j))) return rc;
-  bcgs_init<float><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, h->iR, h->iRP, h->iP, h->iV, st, h->red_partial2);
+  bcgs_init<float><<<bcgs_grid<float>(n), RED_THREADS, 0, h->stream>>>(n, h->iR, h->iRP, h->iP, h->iV, st, h->red_partial2);
   LAUNCHED(h);
   const int vgrid = grid_for(n);
   for (int k = 0; k < h->inner_its; k++) {
     bcgs_p<float><<<vgrid, 256, 0, h->stream>>>(n, h->iR, h->iV, h->iP, st);
     if ((rc = spmv32_pc(h, h->iP, h->iV, nullptr, 0, nullptr, act))) return rc;
-    bcgs_alpha<float><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, h->iV, h->iRP, st, h->red_partial2);
+    bcgs_alpha<float><<<bcgs_grid<float>(n), RED_THREADS, 0, h->stream>>>(n, h->iV, h->iRP, st, h->red_partial2);
     bcgs_s<float><<<vgrid, 256, 0, h->stream>>>(n, h->iR, h->iV, h->iS, st);
     if ((rc = spmv32_pc(h, h->iS, h->iT, nullptr, 0, nullptr, act))) return rc;
-    bcgs_omega<float><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, h->iS, h->iT, st, h->red_partial2);
-    bcgs_xr<float><<<red_grid(n), RED_THREADS, 0, h->stream>>>(n, z, h->iP, h->iS, h->iT, h->iR, h->iRP, st,
+    bcgs_omega<float><<<bcgs_grid<float>(n), RED_THREADS, 0, h->stream>>>(n, h->iS, h->iT, st, h->red_partial2);
+    bcgs_xr<float><<<bcgs_grid<float>(n), RED_THREADS, 0, h->stream>>>(n, z, h->iP, h->iS, h->iT, h->iR, h->iRP, st,
                                                              h->red_partial2);
     h->launches += 5;
   }

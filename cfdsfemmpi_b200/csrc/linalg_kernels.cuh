@@ -77,6 +77,15 @@ __device__ __forceinline__ double block_sum(double v, double *sh)
   return r;
 }
 
+// Sum of an array in shared memory, one entry after another, by one thread.
+__device__ __forceinline__ double sum_in_order(const double *v, unsigned int count)
+{
+  double t = 0.0;
+#pragma unroll 8
+  for (unsigned int k = 0; k < count; k++) t += v[k];
+  return t;
+}
+
 // Returns true in exactly one CTA (the last to arrive), after all CTAs'
 // partials are visible.
 __device__ __forceinline__ bool last_block(unsigned int *counter, unsigned int nblocks)
