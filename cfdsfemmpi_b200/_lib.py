@@ -19,7 +19,7 @@ EXPORTS = [
     "cfdgpu_create", "cfdgpu_destroy", "cfdgpu_last_error", "cfdgpu_step", "cfdgpu_get_solution",
     "cfdgpu_set_solution", "cfdgpu_device_solution", "cfdgpu_stream", "cfdgpu_set_history", "cfdgpu_get_history",
     "cfdgpu_element_matrices", "cfdgpu_set_element_state", "cfdgpu_pattern_info_get", "cfdgpu_export_pattern",
-    "cfdgpu_pattern_build", "cfdgpu_ilu_pattern_build", "cfdgpu_assemble_export", "cfdgpu_solve_export", "cfdgpu_timers", "cfdgpu_launch_count",
+    "cfdgpu_pattern_build", "cfdgpu_ilu_pattern_build", "cfdgpu_trsv_plan_build", "cfdgpu_assemble_export", "cfdgpu_solve_export", "cfdgpu_timers", "cfdgpu_launch_count",
     "cfdgpu_set_profiling", "cfdgpu_kernel_stats", "cfdgpu_true_residual", "cfdgpu_residual_norm_noalloc",
     "cfdgpu_ilu_export", "cfdgpu_pc_apply_export",
     "cfdgpu_mpnn_create", "cfdgpu_mpnn_destroy", "cfdgpu_mpnn_num_params", "cfdgpu_mpnn_get_params",
@@ -91,6 +91,12 @@ class IluInfo(ctypes.Structure):
                 ("chain_levels_l", ctypes.c_int), ("chain_levels_u", ctypes.c_int)]
 
 
+class TrsvInfo(ctypes.Structure):
+    _fields_ = [("warps", ctypes.c_int), ("cap", ctypes.c_int), ("slots_max", ctypes.c_int),
+                ("ngroups", ctypes.c_int64), ("npieces", ctypes.c_int64), ("ndesc", ctypes.c_int64),
+                ("next", ctypes.c_int64)]
+
+
 _LIB: Optional[ctypes.CDLL] = None
 
 
@@ -124,6 +130,7 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     L.cfdgpu_export_pattern.argtypes = [vp] + [vp] * 8
     L.cfdgpu_pattern_build.argtypes = [ctypes.POINTER(Mesh), ctypes.POINTER(PatternInfo)] + [vp] * 8
     L.cfdgpu_ilu_pattern_build.argtypes = [ctypes.POINTER(Mesh), ip, ip, ctypes.POINTER(IluInfo)] + [vp] * 9
+    L.cfdgpu_trsv_plan_build.argtypes = [ctypes.POINTER(Mesh), ip, ip, ip, ctypes.POINTER(TrsvInfo)] + [vp] * 5
     L.cfdgpu_assemble_export.argtypes = [vp, ip, vp, vp]
     L.cfdgpu_solve_export.argtypes = [vp, vp, vp, ctypes.POINTER(ip), ctypes.POINTER(ip)]
     L.cfdgpu_timers.argtypes = [vp, vp]
@@ -250,6 +257,25 @@ def ilu_pattern_build(mesh, levels: int = 0, nblocks: int = 1) -> dict:
     d["uchain"] = d["uchain"][:2 * info.nchains_u].reshape(-1, 2)
     d["lchain_order"] = d["lchain_order"][:info.nchains_l]
     d["uchain_order"] = d["uchain_order"][:info.nchains_u]
+    d["info"] = info
+    return d
+
+
+def trsv_plan_build(mesh, levels: int = 0, nblocks: int = 1, upper: bool = False) -> dict:
+    """Host-only schedule of a triangular solve (cfdgpu_trsv_plan_build); needs no GPU."""
+    L = load()
+    m, keep = _mesh_struct(mesh)
+    info = TrsvInfo()
+    args = (ctypes.byref(m), levels, nblocks, int(upper), ctypes.byref(info))
+    rc = L.cfdgpu_trsv_plan_build(*args, *([None] * 5))
+    if rc != 0:
+        raise CfdGpuError(rc, "triangular-solve schedule build failed")
+    d = {"groups": np.zeros((info.ngroups, 4), np.int32), "wptr": np.zeros((info.ngroups, info.warps + 1), np.int32),
+         "pieces": np.zeros((info.npieces, 4), np.int32), "desc": np.zeros(max(info.ndesc, 1), np.uint32),
+         "ext": np.zeros(max(info.next, 1), np.int32)}
+    rc = L.cfdgpu_trsv_plan_build(*args, *[_ptr(d[k]) for k in ("groups", "wptr", "pieces", "desc", "ext")])
+    if rc != 0:
+        raise CfdGpuError(rc, "triangular-solve schedule build failed")
     d["info"] = info
     return d
 

@@ -117,8 +117,8 @@ struct cfdgpu_handle {
   // block-Jacobi ILU(k) preconditioner (pc_type CFDGPU_PC_BJACOBI_ILU)
   IluPattern ilu;
   int32_t *frow = nullptr, *fcol = nullptr, *fdiag = nullptr, *faslot = nullptr, *fumap = nullptr;
-  int32_t *florder = nullptr, *fuorder = nullptr;
-  int32_t *flchain = nullptr, *fuchain = nullptr, *flchord = nullptr, *fuchord = nullptr, *fperm = nullptr;
+  int32_t *florder = nullptr, *fperm = nullptr;
+  TrsvView plan_l{}, plan_u{};     // schedules of the lower and upper solve
   int64_t *fuoff = nullptr;
   double *fval = nullptr, *fdinv = nullptr;
   unsigned int *iflags = nullptr;
@@ -191,7 +191,8 @@ template <typename T>
 static int dalloc(cfdgpu_handle *h, T **p, size_t count)
 {
   void *q = nullptr;
-  size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
+  // 32 bytes of slack: the triangular solves copy whole 16-byte lines of vectors and factors
+  size_t bytes = std::max<size_t>(count, 1) * sizeof(T) + 32;
   cudaError_t e = cudaMalloc(&q, bytes);
   if (e != cudaSuccess) {
     h->err = std::string("cudaMalloc(") + std::to_string(bytes) + "): " + cudaGetErrorString(e);
@@ -497,26 +498,6 @@ static int ilu_factor_run32(cfdgpu_handle *h)
   return check_launch(h, "ilu_factor32");
 }
 
-// z = (L U)^-1 r with the FP32 factors on FP32 vectors
-static int ilu_apply32(cfdgpu_handle *h, const float *r, float *z, const GmresState *st, int j, const int *active)
-{
-  if ((const void *)r == (const void *)z) { h->err = "ILU apply: input and output overlap"; return CFDGPU_EINVAL; }
-  const int pi = prof_begin(h, CFDGPU_KIND_TRSV, 0.5 * trsv_bytes(h));
-  const int nl = (int)h->ilu.lchain_order.size(), nu = (int)h->ilu.uchain_order.size();
-  // every chain of a wavefront band is in flight at once: up to one warp per chain
-  const int gl = ilu_grid(nl, nl), gu = ilu_grid(nu, nu);
-#define TRSV32(NB)                                                                                              \
-  ilu_trsv<NB, false, float, float><<<gl, ILU_THREADS, 0, h->stream>>>(nl, h->flchord, h->flchain, h->frow,       \
-      h->fcol, h->fdiag, h->fval32, h->fdinv32, h->fperm, r, h->ybuf32, z, h->tctl, st, j, active);                      \
-  ilu_trsv<NB, true, float, float><<<gu, ILU_THREADS, 0, h->stream>>>(nu, h->fuchord, h->fuchain, h->frow,        \
-      h->fcol, h->fdiag, h->fval32, h->fdinv32, h->fperm, nullptr, h->ybuf32, z, h->tctl, st, j, active);
-  if (h->ndof == 4) { TRSV32(4); } else { TRSV32(3); }
-#undef TRSV32
-  prof_end(h, pi);
-  h->launches += 2;
-  return check_launch(h, "ilu_solve32");
-}
-
 // numeric block ILU of the assembled FP64 matrix
 static int ilu_factor_run(cfdgpu_handle *h)
 {
@@ -535,24 +516,71 @@ static int ilu_factor_run(cfdgpu_handle *h)
   return check_launch(h, "ilu_factor");
 }
 
+// Schedule of the lower or upper solve, uploaded.
+static int upload_trsv(cfdgpu_handle *h, bool upper, TrsvView &V)
+{
+  TrsvPlan p;
+  build_trsv_plan(h->ilu, h->ndof, upper, p);
+  TrsvGroup *groups;
+  TrsvPiece *pieces;
+  int32_t *wptr, *ext;
+  uint32_t *desc;
+  int rc;
+  if ((rc = upload(h, &groups, p.groups.data(), p.groups.size())) || (rc = upload(h, &wptr, p.wptr.data(), p.wptr.size())) ||
+      (rc = upload(h, &pieces, p.pieces.data(), p.pieces.size())) || (rc = upload(h, &desc, p.desc.data(), p.desc.size())) ||
+      (rc = upload(h, &ext, p.ext.data(), p.ext.size())))
+    return rc;
+  V.groups = groups; V.wptr = wptr; V.pieces = pieces; V.desc = desc; V.ext = ext;
+  V.ngroups = (int)p.groups.size();
+  V.slots = p.max_slots;
+  return 0;
+}
+
+// One triangular solve (ilu_trsv) on the schedule V: one CTA per SM.
+template <int NB, bool UPPER, typename T>
+static cudaError_t launch_trsv(cfdgpu_handle *h, const TrsvView &V, const T *fval, const T *fdinv, const T *r, T *y, T *z,
+                               const GmresState *st, int j, const int *active)
+{
+  const size_t smem = trsv_smem<NB, UPPER, T>(V.slots);
+  cudaError_t e = cudaFuncSetAttribute(ilu_trsv<NB, UPPER, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  ilu_trsv<NB, UPPER, T><<<std::min(V.ngroups, 148), TRSV_THREADS, smem, h->stream>>>(V, fval, fdinv, h->fperm, r, y, z,
+                                                                                    h->tctl, st, j, active);
+  return cudaGetLastError();
+}
+
 // z = (L U)^-1 r: lower solve r -> y (the handle's buffer), upper solve y -> z
-static int ilu_apply(cfdgpu_handle *h, const double *r, double *z, const GmresState *st, int j, const int *active)
+template <typename T>
+static int ilu_apply_t(cfdgpu_handle *h, const T *fval, const T *fdinv, T *ybuf, const T *r, T *z,
+                       const GmresState *st, int j, const int *active)
 {
   if ((const void *)r == (const void *)z) { h->err = "ILU apply: input and output overlap"; return CFDGPU_EINVAL; }
-  const int pi = prof_begin(h, CFDGPU_KIND_TRSV, trsv_bytes(h));
-  const int nl = (int)h->ilu.lchain_order.size(), nu = (int)h->ilu.uchain_order.size();
-  // every chain of a wavefront band is in flight at once: up to one warp per chain
-  const int gl = ilu_grid(nl, nl), gu = ilu_grid(nu, nu);
-#define TRSV64(NB)                                                                                                \
-  ilu_trsv<NB, false, double, double><<<gl, ILU_THREADS, 0, h->stream>>>(nl, h->flchord, h->flchain, h->frow,       \
-      h->fcol, h->fdiag, h->fval, h->fdinv, h->fperm, r, h->ybuf, z, h->tctl, st, j, active);                              \
-  ilu_trsv<NB, true, double, double><<<gu, ILU_THREADS, 0, h->stream>>>(nu, h->fuchord, h->fuchain, h->frow,        \
-      h->fcol, h->fdiag, h->fval, h->fdinv, h->fperm, nullptr, h->ybuf, z, h->tctl, st, j, active);
-  if (h->ndof == 4) { TRSV64(4); } else { TRSV64(3); }
-#undef TRSV64
+  const int pi = prof_begin(h, CFDGPU_KIND_TRSV, trsv_bytes(h) * (sizeof(T) / 8.0));
+  cudaError_t e;
+  if (h->ndof == 4) {
+    e = launch_trsv<4, false, T>(h, h->plan_l, fval, fdinv, r, ybuf, z, st, j, active);
+    if (e == cudaSuccess) e = launch_trsv<4, true, T>(h, h->plan_u, fval, fdinv, nullptr, ybuf, z, st, j, active);
+  } else {
+    e = launch_trsv<3, false, T>(h, h->plan_l, fval, fdinv, r, ybuf, z, st, j, active);
+    if (e == cudaSuccess) e = launch_trsv<3, true, T>(h, h->plan_u, fval, fdinv, nullptr, ybuf, z, st, j, active);
+  }
   prof_end(h, pi);
   h->launches += 2;
-  return check_launch(h, "ilu_solve");
+  if (e != cudaSuccess) {
+    h->err = std::string("ilu_solve: ") + cudaGetErrorString(e);
+    return CFDGPU_ECUDA;
+  }
+  return 0;
+}
+
+static int ilu_apply(cfdgpu_handle *h, const double *r, double *z, const GmresState *st, int j, const int *active)
+{
+  return ilu_apply_t<double>(h, h->fval, h->fdinv, h->ybuf, r, z, st, j, active);
+}
+
+static int ilu_apply32(cfdgpu_handle *h, const float *r, float *z, const GmresState *st, int j, const int *active)
+{
+  return ilu_apply_t<float>(h, h->fval32, h->fdinv32, h->ybuf32, r, z, st, j, active);
 }
 
 // errors recorded by the ILU kernels since the last check (zero pivot in the
@@ -1304,11 +1332,7 @@ int cfdgpu_create(const cfdgpu_mesh *mesh, const cfdgpu_control *ctrl, const cfd
     if ((rc = upload(h, &h->fuoff, f.uoff.data(), f.uoff.size()))) return rc;
     if ((rc = upload(h, &h->fumap, f.umap.data(), f.umap.size()))) return rc;
     if ((rc = upload(h, &h->florder, f.lorder.data(), f.lorder.size()))) return rc;
-    if ((rc = upload(h, &h->fuorder, f.uorder.data(), f.uorder.size()))) return rc;
-    if ((rc = upload(h, &h->flchain, f.lchain.data(), f.lchain.size()))) return rc;
-    if ((rc = upload(h, &h->fuchain, f.uchain.data(), f.uchain.size()))) return rc;
-    if ((rc = upload(h, &h->flchord, f.lchain_order.data(), f.lchain_order.size()))) return rc;
-    if ((rc = upload(h, &h->fuchord, f.uchain_order.data(), f.uchain_order.size()))) return rc;
+    if ((rc = upload_trsv(h, false, h->plan_l)) || (rc = upload_trsv(h, true, h->plan_u))) return rc;
     if (!f.perm.empty() && (rc = upload(h, &h->fperm, f.perm.data(), f.perm.size()))) return rc;
     if (h->mixed) {
       if ((rc = dalloc(h, &h->fval32, (size_t)f.nnzb() * bb))) return rc;
@@ -1733,6 +1757,31 @@ int cfdgpu_ilu_pattern_build(const cfdgpu_mesh *mesh, int levels, int nblocks, c
     else
       cp(perm, f.perm);
   }
+  return 0;
+}
+
+int cfdgpu_trsv_plan_build(const cfdgpu_mesh *mesh, int levels, int nblocks, int upper, cfdgpu_trsv_info *info,
+                           int32_t *groups, int32_t *wptr, int32_t *pieces, uint32_t *desc, int32_t *ext)
+{
+  if (!mesh || !info || !mesh->conn) return CFDGPU_EINVAL;
+  Topology t;
+  std::string msg = build_topology(mesh->nNode, mesh->nElem, mesh->npElem, mesh->ndim + 1, mesh->conn, mesh->nDBC,
+                                   mesh->dbc_node, mesh->dbc_dof, mesh->dbc_value, t);
+  if (!msg.empty()) return CFDGPU_EINVAL;
+  IluPattern f;
+  msg = build_ilu_pattern(t, levels, nblocks, f);
+  if (!msg.empty()) return CFDGPU_EINVAL;
+  TrsvPlan p;
+  build_trsv_plan(f, t.ndof, upper != 0, p);
+  info->warps = TRSV_WARPS;
+  info->cap = trsv_cap(t.ndof);
+  info->slots_max = trsv_max_slots(t.ndof);
+  info->ngroups = (int64_t)p.groups.size();
+  info->npieces = (int64_t)p.pieces.size();
+  info->ndesc = (int64_t)p.desc.size();
+  info->next = (int64_t)p.ext.size();
+  auto cp = [](auto *dst, const auto &v) { if (dst && !v.empty()) memcpy(dst, v.data(), v.size() * sizeof(v[0])); };
+  cp(groups, p.groups); cp(wptr, p.wptr); cp(pieces, p.pieces); cp(desc, p.desc); cp(ext, p.ext);
   return 0;
 }
 

@@ -233,6 +233,30 @@ int cfdgpu_ilu_pattern_build(const cfdgpu_mesh *mesh, int levels, int nblocks, c
                              int32_t *rowptr, int32_t *colidx, int32_t *perm, int32_t *lorder, int32_t *uorder,
                              int32_t *lchain, int32_t *uchain, int32_t *lchain_order, int32_t *uchain_order);
 
+/* Host-only: the schedule of the lower (upper = 0) or upper (1) triangular
+ * solve: groups of rows handed to CTAs in this order, the pieces (at most
+ * cap blocks of one row) of each of a group's warps, and the slots in shared
+ * memory where a group keeps its rows' values and its inputs.  Call once with
+ * NULL arrays to get the sizes, then with arrays of those sizes: groups
+ * (4 x ngroups: rows, first input, inputs, the
+ * input that the group starts with), wptr (ngroups x (warps + 1):
+ * pieces of each warp), pieces (4 x npieces: first factor block, blocks |
+ * 1 << 16 on a row's first and | 1 << 17 on its last piece | low bits of the
+ * first block << 18, first entry of its record / 4, node (lower) or factor row
+ * (upper)), desc (ndesc: per piece a record of factor row, node, the second
+ * entry again, the row's own slot | that of the block nearest the diagonal
+ * << 16 (in doubles), then byte offsets of the blocks' slots: the q-th block's
+ * is entry 4 (q mod s) + q / s, s = 4 for 4x4 and 8 for 3x3 blocks, of 4 s; with
+ * 1 << 20 in the second entry, positions in the source vector instead), ext
+ * (next: factor rows).  Used by tests to check that every input of a row
+ * is its group's or an earlier group's, on which the kernel's progress rests. */
+typedef struct cfdgpu_trsv_info {
+  int warps, cap, slots_max;   /* solving warps per group, blocks per piece, largest group allowed */
+  int64_t ngroups, npieces, ndesc, next;
+} cfdgpu_trsv_info;
+int cfdgpu_trsv_plan_build(const cfdgpu_mesh *mesh, int levels, int nblocks, int upper, cfdgpu_trsv_info *info,
+                           int32_t *groups, int32_t *wptr, int32_t *pieces, uint32_t *desc, int32_t *ext);
+
 /* Assemble (iteration-0 semantics when iter == 0: lifting included) at the
  * current state and copy the BSR values (nnzb*ndof*ndof, FP64, block
  * row-major) and the RHS (nNode*ndof) to host.  Uses the td[] of the last
