@@ -116,7 +116,9 @@ struct cfdgpu_handle {
   double prof_bytes[CFDGPU_KIND_COUNT] = {};
   // block-Jacobi ILU(k) preconditioner (pc_type CFDGPU_PC_BJACOBI_ILU)
   IluPattern ilu;
-  int32_t *frow = nullptr, *fcol = nullptr, *fdiag = nullptr, *faslot = nullptr, *fumap = nullptr;
+  int32_t *frow = nullptr, *fcol = nullptr, *fdiag = nullptr, *faslot = nullptr;
+  uint32_t *fumap = nullptr;
+  double *frowbuf = nullptr;       // factorisation rows that do not fit into shared memory
   int32_t *florder = nullptr, *fperm = nullptr;
   TrsvView plan_l{}, plan_u{};     // schedules of the lower and upper solve
   int64_t *fuoff = nullptr;
@@ -451,25 +453,12 @@ static int assemble(cfdgpu_handle *h, int iter, bool want_K)
   return 0;
 }
 
-// Persistent grid of the sync-free ILU kernels: warps in flight for `tasks`
-// rows whose widest dependency level holds `width` rows.  Warps beyond what
-// the levels can feed only add polling traffic: on the 115^3 cavity the
-// triangular-solve pair takes 5.4 ms with 2 CTAs of 8 warps per SM against
-// 9.5 ms with 4 and 14 ms with 8, and a chain of single-row levels (the
-// complete factorisation of a band) needs a few dozen warps, not thousands.
-static inline int ilu_grid(int64_t tasks, int64_t width)
-{
-  const int64_t warps = std::min<int64_t>(tasks, std::max<int64_t>(256, 2 * width));
-  const int64_t ctas = (warps + ILU_WARPS - 1) / ILU_WARPS;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(ctas, 148 * 2));
-}
-
 static double ilu_factor_bytes(cfdgpu_handle *h)
 {
   // read A and the update map once, write the factors and the inverted diagonals once
   const double bb = (double)h->ndof * h->ndof * 8.0;
   return (double)h->topo.nnzb() * bb + (double)h->ilu.nnzb() * bb + (double)h->nNode * bb +
-         4.0 * (double)h->ilu.umap.size();
+         4.0 * (double)h->ilu.umap.size() + 8.0 * (double)h->ilu.uoff.size();
 }
 
 static double trsv_bytes(cfdgpu_handle *h)
@@ -480,40 +469,51 @@ static double trsv_bytes(cfdgpu_handle *h)
   return (double)h->ilu.nnzb() * (bb + 4.0) + (double)h->nNode * bb + 4.0 * V;
 }
 
-// numeric block ILU of the FP32 copy (mixed mode: FP64 arithmetic, FP32 factors)
-static int ilu_factor_run32(cfdgpu_handle *h)
+// Shared memory for one warp's row of the factorisation, warps per CTA and
+// CTAs: as many warps as the rows leave room for (8 at most, two CTAs per SM),
+// and no more than twice the widest dependency level holds (at least 256), since
+// warps beyond what the levels can feed only add polling traffic.
+struct FactorLaunch {
+  int warps, grid;
+  size_t smem;
+  bool in_smem;
+};
+static FactorLaunch factor_launch(cfdgpu_handle *h)
 {
-  const int pi = prof_begin(h, CFDGPU_KIND_ILU, 0.5 * ilu_factor_bytes(h));
-  const int grid = ilu_grid(h->nNode, h->ilu.maxw_l);
-  if (h->ndof == 4)
-    ilu_factor<4, float, float><<<grid, ILU_THREADS, 0, h->stream>>>(h->nNode, h->rowptr, h->faslot, h->bsr32, h->frow,
-                                                                    h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder, h->fperm,
-                                                                    h->fval32, h->fdinv32, h->iflags, h->tctl);
-  else
-    ilu_factor<3, float, float><<<grid, ILU_THREADS, 0, h->stream>>>(h->nNode, h->rowptr, h->faslot, h->bsr32, h->frow,
-                                                                    h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder, h->fperm,
-                                                                    h->fval32, h->fdinv32, h->iflags, h->tctl);
-  prof_end(h, pi);
-  LAUNCHED(h);
-  return check_launch(h, "ilu_factor32");
+  constexpr size_t PER_SM = 220 * 1024;
+  const size_t row = (size_t)h->ilu.maxrow * h->ndof * h->ndof * sizeof(double);
+  FactorLaunch f;
+  f.in_smem = row <= PER_SM;
+  f.warps = f.in_smem ? (int)std::min<size_t>(ILU_WARPS, PER_SM / row) : ILU_WARPS;
+  f.smem = f.in_smem ? f.warps * row : 0;
+  const int per_sm = f.smem <= PER_SM / 2 ? 2 : 1;
+  const int64_t want = std::min<int64_t>(h->nNode, std::max<int64_t>(256, 2 * (int64_t)h->ilu.maxw_l));
+  f.grid = (int)std::max<int64_t>(1, std::min<int64_t>((want + f.warps - 1) / f.warps, 148 * per_sm));
+  return f;
 }
 
-// numeric block ILU of the assembled FP64 matrix
-static int ilu_factor_run(cfdgpu_handle *h)
+// numeric block ILU of the assembled matrix (FP64, or its FP32 copy in mixed mode: FP64 arithmetic, FP32 factors)
+template <int NB, typename T>
+static int ilu_factor_t(cfdgpu_handle *h, const T *a, T *fval, T *fdinv)
 {
-  const int pi = prof_begin(h, CFDGPU_KIND_ILU, ilu_factor_bytes(h));
-  const int grid = ilu_grid(h->nNode, h->ilu.maxw_l);
-  if (h->ndof == 4)
-    ilu_factor<4, double, double><<<grid, ILU_THREADS, 0, h->stream>>>(h->nNode, h->rowptr, h->faslot, h->bsr, h->frow,
-                                                                      h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder, h->fperm,
-                                                                      h->fval, h->fdinv, h->iflags, h->tctl);
-  else
-    ilu_factor<3, double, double><<<grid, ILU_THREADS, 0, h->stream>>>(h->nNode, h->rowptr, h->faslot, h->bsr, h->frow,
-                                                                      h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder, h->fperm,
-                                                                      h->fval, h->fdinv, h->iflags, h->tctl);
+  const int pi = prof_begin(h, CFDGPU_KIND_ILU, ilu_factor_bytes(h) * (sizeof(T) / 8.0));
+  const FactorLaunch f = factor_launch(h);
+  CK(cudaFuncSetAttribute(ilu_factor<NB, T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
+  ilu_factor<NB, T, T><<<f.grid, 32 * f.warps, f.smem, h->stream>>>(
+      h->nNode, h->ilu.maxrow, h->rowptr, h->faslot, a, h->frow, h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder,
+      h->fperm, fval, fdinv, h->iflags, h->tctl, h->frowbuf);
   prof_end(h, pi);
   LAUNCHED(h);
   return check_launch(h, "ilu_factor");
+}
+
+static int ilu_factor_run(cfdgpu_handle *h)
+{
+  if (h->mixed)
+    return h->ndof == 4 ? ilu_factor_t<4, float>(h, h->bsr32, h->fval32, h->fdinv32)
+                        : ilu_factor_t<3, float>(h, h->bsr32, h->fval32, h->fdinv32);
+  return h->ndof == 4 ? ilu_factor_t<4, double>(h, h->bsr, h->fval, h->fdinv)
+                      : ilu_factor_t<3, double>(h, h->bsr, h->fval, h->fdinv);
 }
 
 // Schedule of the lower or upper solve, uploaded.
@@ -610,7 +610,7 @@ static int build_pc(cfdgpu_handle *h)
 {
   const int pc = h->opts.pc_type;
   if (pc == CFDGPU_PC_NONE) return 0;
-  if (pc == CFDGPU_PC_BJACOBI_ILU) return h->mixed ? ilu_factor_run32(h) : ilu_factor_run(h);
+  if (pc == CFDGPU_PC_BJACOBI_ILU) return ilu_factor_run(h);
   const int g = (h->nNode + 127) / 128;
   if (h->mixed && h->ndof == 4) {
     build_jacobi<4, float, float><<<g, 128, 0, h->stream>>>(h->nNode, h->diag_slot, h->bsr32, h->dinv32, h->binv32, pc);
@@ -1344,6 +1344,10 @@ int cfdgpu_create(const cfdgpu_mesh *mesh, const cfdgpu_control *ctrl, const cfd
       CK(cudaMemset(h->fval, 0, sizeof(double) * f.nnzb() * bb));
       if ((rc = dalloc(h, &h->fdinv, (size_t)h->nNode * bb))) return rc;
       CK(cudaMemset(h->fdinv, 0, sizeof(double) * h->nNode * bb));
+    }
+    {
+      const FactorLaunch fl = factor_launch(h);
+      if (!fl.in_smem && (rc = dalloc(h, &h->frowbuf, (size_t)fl.grid * fl.warps * f.maxrow * bb))) return rc;
     }
     if ((rc = dalloc(h, &h->iflags, (size_t)h->nNode))) return rc;
     CK(cudaMemset(h->iflags, 0, sizeof(unsigned int) * h->nNode));

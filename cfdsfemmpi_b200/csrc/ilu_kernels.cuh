@@ -12,9 +12,8 @@
 // Scheduling is sync-free.  Factorisation: one persistent grid whose warps draw
 // rows from an atomic ticket in level-set order (computed on the host).  Rows of
 // one level are independent, so a row only waits for rows handed out before it:
-// a row whose inputs are not ready polls their flags (relaxed loads with
-// back-off, then one acquire fence), and a finished row publishes its flag with
-// a release store.  Triangular solves: persistent CTAs draw groups of rows
+// a row whose inputs are not ready polls their flags (acquire loads with
+// back-off), and a finished row publishes its flag after a fence.  Triangular solves: persistent CTAs draw groups of rows
 // (trsv_plan.h), and the solved values are their own ready flags.  The earliest
 // unfinished row always has its inputs, so progress is guaranteed; every wait
 // is bounded and records a time-out in the control block instead of spinning
@@ -62,36 +61,24 @@ __device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int *p)
   return v;
 }
 
-__device__ __forceinline__ void st_release_u32(unsigned int *p, unsigned int v)
+__device__ __forceinline__ void st_relaxed_u32(unsigned int *p, unsigned int v)
 {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int *p)
-{
-  unsigned int v;
-  asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-__device__ __forceinline__ void fence_acq_rel_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
-// Wait until *f == target (bounded): relaxed polls, the first ILU_SPIN_HOT_POLLS
-// back to back, then with exponential back-off.
-// The caller completes the acquire with fence_acq_rel_gpu() after the polls
-// of all its lanes (one fence per row instead of one acquire per input).
+// Wait (a whole warp on one flag, bounded) until *f == target: acquire loads,
+// the first ILU_SPIN_HOT_POLLS back to back, then with exponential back-off.
 // Returns false after a time-out, or when another warp has already timed out.
 __device__ __forceinline__ bool wait_flag(const unsigned int *f, unsigned int target, TriCtl *ctl)
 {
-  if (ld_relaxed_u32(f) == target) return true;
   unsigned int ns = 32;
   for (int it = 0; it < ILU_SPIN_LIMIT; it++) {
+    if (ld_acquire_u32(f) == target) return true;
     if (it >= ILU_SPIN_HOT_POLLS) {
       __nanosleep(ns);
       if (ns < 1024) ns <<= 1;
+      if (*(volatile unsigned int *)&ctl->error) return false;
     }
-    if (ld_relaxed_u32(f) == target) return true;
-    if (*(volatile unsigned int *)&ctl->error) return false;
   }
   atomicCAS(&ctl->error, 0u, ILU_ERR_TIMEOUT);
   return false;
@@ -122,153 +109,206 @@ __device__ __forceinline__ void launch_done(TriCtl *ctl, int lane, unsigned int 
   }
 }
 
-template <typename T>
-__device__ __forceinline__ double ld_cg(const T *p)
+// NB entries at p (a row of a block) past L1: other SMs write them
+template <int NB, typename T>
+__device__ __forceinline__ void ld_row(const T *p, double (&v)[NB])
 {
-  return (double)__ldcg(p);
+  if constexpr (NB == 4 && sizeof(T) == 8) {
+    const double2 a = __ldcg(reinterpret_cast<const double2 *>(p)), b = __ldcg(reinterpret_cast<const double2 *>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  } else if constexpr (NB == 4) {
+    const float4 a = __ldcg(reinterpret_cast<const float4 *>(p));
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  } else {
+#pragma unroll
+    for (int c = 0; c < NB; c++) v[c] = (double)__ldcg(p + c);
+  }
 }
 
-// Invert an NB x NB block (row-major, FP64) with partial pivoting; returns
-// false when a pivot column is zero.
+// Inverse of the NB x NB block at A (row-major) by a warp: Gauss-Jordan with
+// partial pivoting on [A | I], lane = (row, column) of its NB x 2 NB entries.
+// Returns the lane's entry of the inverse (lanes with column >= NB); ok is
+// false (in every lane) when a pivot column is zero.
 template <int NB>
-__device__ __forceinline__ bool invert_block(double (&A)[NB][NB], double (&I)[NB][NB])
+__device__ __forceinline__ double invert_block(const double *A, int lane, bool &ok)
 {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int C = 2 * NB;
+  const int r = lane / C < NB ? lane / C : 0, c = lane % C;
+  double v = c < NB ? A[r * NB + c] : (c - NB == r ? 1.0 : 0.0);
+  ok = true;
 #pragma unroll
-  for (int a = 0; a < NB; a++)
+  for (int k = 0; k < NB; k++) {
+    double col[NB];
 #pragma unroll
-    for (int c = 0; c < NB; c++) I[a][c] = (a == c) ? 1.0 : 0.0;
-  bool ok = true;
+    for (int q = 0; q < NB; q++) col[q] = __shfl_sync(FULL, v, q * C + k);
+    int piv = k;
+    double best = col[k];
 #pragma unroll
-  for (int c = 0; c < NB; c++) {
-    int piv = c;
+    for (int q = k + 1; q < NB; q++)
+      if (fabs(col[q]) > fabs(best)) { piv = q; best = col[q]; }
+    if (best == 0.0) ok = false;
+    const double d = best != 0.0 ? 1.0 / best : 0.0;
+    // rows k and piv change places
+    const int from = r == k ? piv : r == piv ? k : r;
+    double f = from == k ? col[k] : best;     // entry (r, k) after that
 #pragma unroll
-    for (int r = c + 1; r < NB; r++)
-      if (fabs(A[r][c]) > fabs(A[piv][c])) piv = r;
-    if (A[piv][c] == 0.0) ok = false;
-#pragma unroll
-    for (int k = 0; k < NB; k++) {
-      if (piv != c) {
-        double t = A[c][k]; A[c][k] = A[piv][k]; A[piv][k] = t;
-        t = I[c][k]; I[c][k] = I[piv][k]; I[piv][k] = t;
-      }
-    }
-    const double p = A[c][c];
-    const double d = (p != 0.0) ? 1.0 / p : 0.0;
-#pragma unroll
-    for (int k = 0; k < NB; k++) { A[c][k] *= d; I[c][k] *= d; }
-#pragma unroll
-    for (int r = 0; r < NB; r++) {
-      if (r == c) continue;
-      const double f = A[r][c];
-#pragma unroll
-      for (int k = 0; k < NB; k++) { A[r][k] -= f * A[c][k]; I[r][k] -= f * I[c][k]; }
-    }
+    for (int q = 0; q < NB; q++)
+      if (q == r && q != k && q != piv) f = col[q];
+    v = __shfl_sync(FULL, v, from * C + c);
+    const double top = __shfl_sync(FULL, v, k * C + c) * d;
+    v = r == k ? top : v - f * top;
   }
-  return ok;
+  return v;
 }
 
 // ---------------------------------------------------------------------------
-// Numeric block ILU: one warp per node row, rows in ascending order.  For row
-// i: W = the row of A on the factor pattern (fill blocks zero); for every
-// pivot p < i of the row in increasing column order, L_ip = W_p U_pp^-1 and
+// Numeric block ILU: one warp per node row, rows in level order.  For row i:
+// W = the row of A on the factor pattern (fill blocks zero); for every pivot
+// p < i of the row in increasing column order, L_ip = W_p U_pp^-1 and
 // W_j -= L_ip U_pj for the blocks j > p of row p that lie in row i's pattern
-// (their positions come from the symbolic phase's update map); then
-// U_ii^-1.  AT is the type of the assembled matrix, FT of the factors
-// (FP64 arithmetic in both cases).
+// (list umap: the block's number in row p after the diagonal, and its place in
+// row i); then U_ii^-1.  AT is the type of the assembled matrix, FT of the
+// factors; W is FP64 and lives in shared memory (in `scratch` when a row does
+// not fit).
+//
+// What bounds it: the dependency chain, per level the last pivot's hop.  With W
+// in global memory, one fence per pivot and the inverse by one lane the kernel
+// took 8.1 ms at 64^3 (hex8, ILU(0), 455 levels: 18 us each), 3.6 at 32^3, 0.58 at
+// 11^3, 13.9 ms on the 256 x 128 O-grid with ILU(3) (1,404 levels) and 55.7 ms for
+// the complete LU of the 64 x 64 cavity (4,224 levels).  Now a pivot's inverse and
+// the blocks of its row are requested together once its flag is seen (pivots long
+// done are found by one poll of all flags), and the row's blocks that others need
+// are written and published before the rest: 3.5, 1.5, 0.25, 4.5 and 24.1 ms (FP32
+// values are rounded where they were stored before, so the factors keep their bits).
 template <int NB, typename AT, typename FT>
-__global__ void __launch_bounds__(ILU_THREADS)
-ilu_factor(int n, const int32_t *__restrict__ arow, const int32_t *__restrict__ aslot, const AT *__restrict__ aval,
-           const int32_t *__restrict__ fptr, const int32_t *__restrict__ fcol, const int32_t *__restrict__ fdiag,
-           const int64_t *__restrict__ uoff, const int32_t *__restrict__ umap, const int32_t *__restrict__ order,
-           const int32_t *__restrict__ perm, FT *fval, FT *fdinv, unsigned int *flags, TriCtl *ctl)
+__global__ void __launch_bounds__(ILU_THREADS, 2)
+ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *__restrict__ aslot,
+           const AT *__restrict__ aval, const int32_t *__restrict__ fptr, const int32_t *__restrict__ fcol,
+           const int32_t *__restrict__ fdiag, const int64_t *__restrict__ uoff, const uint32_t *__restrict__ umap,
+           const int32_t *__restrict__ order, const int32_t *__restrict__ perm, FT *fval, FT *fdinv,
+           unsigned int *flags, TriCtl *ctl, double *scratch)
 {
   constexpr int BB = NB * NB;
-  constexpr int G = 32 / BB;          // blocks per warp step
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  constexpr int PER = 32 / NB;        // blocks updated at once: lane = (block, row)
+  constexpr int UNR = 2;
+  extern __shared__ __align__(16) double wsm[];
   __shared__ double Lsh[ILU_WARPS][BB];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double *const W = scratch ? scratch + (int64_t)(blockIdx.x * (blockDim.x / 32) + w) * rowcap * BB
+                            : wsm + (int64_t)w * rowcap * BB;
   const unsigned int epoch = *(volatile unsigned int *)&ctl->epoch;
   const unsigned int target = epoch + 1u;
-  const int g = lane / BB, e = lane % BB, er = e / NB, ec = e % NB;
+  const int e = lane % BB, er = e / NB, ec = e % NB;
+  const int ob = lane / NB, orow = lane % NB;
   while (true) {
     const int tk = draw_ticket(ctl, lane);
     if (tk >= n) break;
     const int i = order[tk];
     const int f0 = fptr[i], f1 = fptr[i + 1], fd = fdiag[i];
-    for (int64_t x = (int64_t)f0 * BB + lane; x < (int64_t)f1 * BB; x += 32) fval[x] = FT(0);
+    for (int x = lane; x < (f1 - f0) * BB; x += 32) W[x] = 0.0;
     __syncwarp();
     {
       const int ai = perm ? perm[i] : i;   // node of factor row i
       const int a0 = arow[ai], a1 = arow[ai + 1];
-      for (int64_t x = lane; x < (int64_t)(a1 - a0) * BB; x += 32) {
-        const int k = a0 + (int)(x / BB);
-        const int s = aslot[k];
-        if (s >= 0) fval[(int64_t)s * BB + x % BB] = (FT)aval[(int64_t)k * BB + x % BB];
+      for (int x = lane; x < (a1 - a0) * BB; x += 32) {
+        const int s = aslot[a0 + x / BB];
+        if (s >= 0) W[(s - f0) * BB + x % BB] = (double)(FT)aval[(int64_t)a0 * BB + x];
       }
     }
     __syncwarp();
+    unsigned done = 0;       // pivots of the current 32 whose flags have been seen
+    int pl = 0;
+    int64_t ul = 0, un = 0;  // this lane's pivot: column, its list
     for (int q = f0; q < fd; q++) {
-      const int p = fcol[q];
-      if (lane == 0) wait_flag(flags + p, target, ctl);
-      __syncwarp();
-      fence_acq_rel_gpu();
-      if (lane < BB) {
+      const int b = (q - f0) & 31;
+      if (b == 0) {
+        const bool in = q + lane < fd;
+        pl = in ? fcol[q + lane] : 0;
+        ul = in ? uoff[q + lane] : 0;
+        un = in ? uoff[q + lane + 1] : 0;
+        done = __ballot_sync(0xffffffffu, in && ld_acquire_u32(flags + pl) == target);
+        __syncwarp();
+      }
+      const int p = __shfl_sync(0xffffffffu, pl, b);
+      const int64_t o0 = __shfl_sync(0xffffffffu, ul, b), o1 = __shfl_sync(0xffffffffu, un, b);
+      const int u0 = fdiag[p] + 1;
+      // this lane's first blocks: entries of the list do not depend on the pivot's values
+      uint32_t ent[UNR];
+#pragma unroll
+      for (int k = 0; k < UNR; k++) {
+        const int64_t o = o0 + k * PER + ob;
+        ent[k] = ob < PER && o < o1 ? umap[o] : 0xffffffffu;
+      }
+      if (!((done >> b) & 1u)) {
+        wait_flag(flags + p, target, ctl);
+        __syncwarp();
+        const int x = q - b + lane;
+        done = __ballot_sync(0xffffffffu, x < fd && ld_acquire_u32(flags + pl) == target);
+        __syncwarp();
+      }
+      double dcol[NB], ub[UNR][NB][NB];
+#pragma unroll
+      for (int k = 0; k < NB; k++) dcol[k] = (double)__ldcg(fdinv + (int64_t)p * BB + k * NB + ec);
+      auto fetch = [&](int k) {
+        if (ent[k] != 0xffffffffu) {
+#pragma unroll
+          for (int c = 0; c < NB; c++) ld_row<NB>(fval + (int64_t)(u0 + (int)(ent[k] >> 16)) * BB + c * NB, ub[k][c]);
+        }
+      };
+#pragma unroll
+      for (int k = 0; k < UNR; k++) fetch(k);
+      {
         double s = 0.0;
 #pragma unroll
-        for (int k = 0; k < NB; k++)
-          s = fma((double)fval[(int64_t)q * BB + er * NB + k], ld_cg(fdinv + (int64_t)p * BB + k * NB + ec), s);
-        Lsh[w][lane] = s;
+        for (int k = 0; k < NB; k++) s = fma(W[(q - f0) * BB + er * NB + k], dcol[k], s);
+        if (lane < BB) Lsh[w][lane] = s;
       }
       __syncwarp();
-      if (lane < BB) fval[(int64_t)q * BB + lane] = (FT)Lsh[w][lane];
-      const int u0 = fdiag[p] + 1, u1 = fptr[p + 1];
-      const int32_t *__restrict__ map = umap + uoff[q] - u0;
+      if (lane < BB) W[(q - f0) * BB + lane] = Lsh[w][lane];
       double lrow[NB];
 #pragma unroll
-      for (int k = 0; k < NB; k++) lrow[k] = Lsh[w][er * NB + k];
-      // UNR independent blocks per lane group in flight: all loads first,
-      // then the updates (each target block is written by one lane group)
-      constexpr int UNR = 4;
-      for (int t0 = u0; t0 < u1; t0 += G * UNR) {
-        int pos[UNR];
-        double ub[UNR][NB];
+      for (int k = 0; k < NB; k++) lrow[k] = Lsh[w][orow * NB + k];
+      for (int64_t o = o0; o < o1; o += PER * UNR) {
 #pragma unroll
-        for (int r = 0; r < UNR; r++) {
-          const int t = t0 + r * G + g;
-          pos[r] = (g < G && t < u1) ? map[t] : -1;
+        for (int k = 0; k < UNR; k++) {
+          if (ent[k] != 0xffffffffu) {
+            double *const t = W + (ent[k] & 0xffffu) * BB + orow * NB;
 #pragma unroll
-          for (int k = 0; k < NB; k++)
-            ub[r][k] = (pos[r] >= 0) ? ld_cg(fval + (int64_t)t * BB + k * NB + ec) : 0.0;
-        }
+            for (int c = 0; c < NB; c++) {
+              double s = 0.0;
 #pragma unroll
-        for (int r = 0; r < UNR; r++) {
-          if (pos[r] >= 0) {
-            double s = 0.0;
-#pragma unroll
-            for (int k = 0; k < NB; k++) s = fma(lrow[k], ub[r][k], s);
-            fval[(int64_t)pos[r] * BB + e] = (FT)((double)fval[(int64_t)pos[r] * BB + e] - s);
+              for (int z = 0; z < NB; z++) s = fma(lrow[z], ub[k][z][c], s);
+              t[c] = (double)(FT)(t[c] - s);   // as stored
+            }
           }
+        }
+        if (o + PER * UNR < o1) {
+#pragma unroll
+          for (int k = 0; k < UNR; k++) {
+            const int64_t x = o + PER * (UNR + k) + ob;
+            ent[k] = ob < PER && x < o1 ? umap[x] : 0xffffffffu;
+          }
+#pragma unroll
+          for (int k = 0; k < UNR; k++) fetch(k);
         }
       }
       __syncwarp();
     }
-    if (lane == 0) {
-      double A[NB][NB], I[NB][NB];
-#pragma unroll
-      for (int a = 0; a < NB; a++)
-#pragma unroll
-        for (int c = 0; c < NB; c++) A[a][c] = (double)fval[(int64_t)fd * BB + a * NB + c];
-      if (!invert_block<NB>(A, I)) {
-        if (atomicCAS(&ctl->error, 0u, ILU_ERR_ZERO_PIVOT) == 0u) ctl->zero_pivot_row = i;
-      }
-#pragma unroll
-      for (int a = 0; a < NB; a++)
-#pragma unroll
-        for (int c = 0; c < NB; c++) fdinv[(int64_t)i * BB + a * NB + c] = (FT)I[a][c];
+    {
+      bool ok;
+      const double v = invert_block<NB>(W + (fd - f0) * BB, lane, ok);
+      if (!ok && lane == 0 && atomicCAS(&ctl->error, 0u, ILU_ERR_ZERO_PIVOT) == 0u) ctl->zero_pivot_row = i;
+      const int r = lane / (2 * NB), c = lane % (2 * NB) - NB;
+      if (r < NB && c >= 0) fdinv[(int64_t)i * BB + r * NB + c] = (FT)v;
     }
-    // every lane's writes of the row are visible before the flag
+    // what later rows read, the flag, then the multipliers
+    for (int x = (fd + 1 - f0) * BB + lane; x < (f1 - f0) * BB; x += 32) fval[(int64_t)f0 * BB + x] = (FT)W[x];
     __threadfence();
     __syncwarp();
-    if (lane == 0) st_release_u32(flags + i, target);
+    if (lane == 0) st_relaxed_u32(flags + i, target);
+    for (int x = lane; x < (fd + 1 - f0) * BB; x += 32) fval[(int64_t)f0 * BB + x] = (FT)W[x];
+    __syncwarp();
   }
   launch_done(ctl, lane, epoch);
 }

@@ -330,27 +330,28 @@ std::string build_ilu_pattern(const Topology &t, int levels, int nblocks, IluPat
     chains(false, f.lchain, f.lchain_order, f.lchain_levels, f.lchain_maxw);
     chains(true, f.uchain, f.uchain_order, f.uchain_levels, f.uchain_maxw);
   }
-  // update map: positions in row i of the upper blocks of every pivot row
+  // update lists: the upper blocks of every pivot row that row i's pattern holds
   {
-    int64_t total = 0;
-    f.uoff.assign(f.colidx.size(), -1);
+    for (int i = 0; i < n; i++) f.maxrow = std::max(f.maxrow, f.rowptr[i + 1] - f.rowptr[i]);
+    if (f.maxrow > 65535) return "ILU row of more than 65535 blocks";
+    f.uoff.resize(f.colidx.size() + 1);
+    int64_t most = 0;
     for (int i = 0; i < n; i++)
-      for (int q = f.rowptr[i]; q < f.diag[i]; q++) {
-        const int p = f.colidx[q];
-        f.uoff[q] = total;
-        total += f.rowptr[p + 1] - f.diag[p] - 1;
-      }
-    f.umap.resize(total);
+      for (int q = f.rowptr[i]; q < f.diag[i]; q++) most += f.rowptr[f.colidx[q] + 1] - f.diag[f.colidx[q]] - 1;
+    f.umap.reserve((size_t)most);
     std::vector<int32_t> pos(n, -1);
     for (int i = 0; i < n; i++) {
-      for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = k;
-      for (int q = f.rowptr[i]; q < f.diag[i]; q++) {
-        const int p = f.colidx[q];
-        int64_t o = f.uoff[q];
-        for (int u = f.diag[p] + 1; u < f.rowptr[p + 1]; u++) f.umap[o++] = pos[f.colidx[u]];
+      for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = k - f.rowptr[i];
+      for (int q = f.rowptr[i]; q < f.rowptr[i + 1]; q++) {
+        f.uoff[q] = (int64_t)f.umap.size();
+        if (q >= f.diag[i]) continue;
+        const int p = f.colidx[q], u0 = f.diag[p] + 1;
+        for (int u = u0; u < f.rowptr[p + 1]; u++)
+          if (pos[f.colidx[u]] >= 0) f.umap.push_back((uint32_t)(u - u0) << 16 | (uint32_t)pos[f.colidx[u]]);
       }
       for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = -1;
     }
+    f.uoff[f.colidx.size()] = (int64_t)f.umap.size();
   }
   // blocks of A inside the factor pattern (A's block (v, c) lands in factor
   // row IP(v) at column IP(c))

@@ -66,11 +66,13 @@ struct IluPattern {
   // which bounds its fill by the graph's bandwidth (a direct solve's result
   // does not depend on the order beyond rounding)
   std::vector<int32_t> perm, iperm;
-  // update map of the numeric factorisation: for a strictly lower block q =
-  // (i, p), umap[uoff[q] + k] is the position in row i of the k-th block
-  // right of the diagonal in row p, or -1 when row i's pattern drops it
-  std::vector<int64_t> uoff;     // nnzb (meaningful for strictly lower blocks)
-  std::vector<int32_t> umap;
+  // updates of the numeric factorisation: for a strictly lower block q = (i, p),
+  // umap[uoff[q]..uoff[q+1]) lists the blocks of row p right of its diagonal that
+  // lie in row i's pattern: their number after the diagonal << 16 | their place
+  // in row i
+  std::vector<int64_t> uoff;     // nnzb + 1
+  std::vector<uint32_t> umap;
+  int maxrow = 0;                // blocks of the longest row
   // rows sorted by level of the lower DAG (factorisation and lower solve:
   // level(i) = 1 + max level of the strictly lower blocks' columns) and of
   // the upper DAG (upper solve), row order inside a level
