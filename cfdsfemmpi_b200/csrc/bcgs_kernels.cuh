@@ -85,13 +85,6 @@ __device__ __forceinline__ void pair_fma(Pair &acc, double x, double y)
   acc = pair_add(acc, {p, fma(x, y, -p)});
 }
 
-// CTAs of a reduction over n entries: four entries per thread, at most RED_BLOCKS
-inline int red_grid(int64_t n)
-{
-  const int64_t g = (n + 4 * RED_THREADS - 1) / (4 * RED_THREADS);
-  return (int)(g < 1 ? 1 : g > RED_BLOCKS ? RED_BLOCKS : g);
-}
-
 // FP32 vectors (the inner solves of the mixed-precision path) have products that
 // are exact in 64 bits and a tolerance of a digit or two: plain sums, and always in
 // the same order (RED_BLOCKS CTAs, their partials one after another), because the

@@ -660,10 +660,10 @@ static int spmv_pc(cfdgpu_handle *h, int mode, const double *x, const double *b,
     }
 #undef SPMV4
   } else {
-    const int grid = (int)((h->n + 255) / 256);
-#define SPMV3(MO, PCV)                                                                                        \
-  bsr_spmv_generic<3, MO, PCV, double><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr, x, b, \
-                                                                     h->dinv, h->binv, y, st, j, xscale, active)
+    const int grid = (int)((h->nNode * 32LL + 255) / 256);
+#define SPMV3(MO, PCV)                                                                                         \
+  bsr3_spmv<MO, PCV, double, double><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr, x, b, \
+                                                                  h->dinv, h->binv, y, st, j, xscale, active)
     if (mode == 0) {
       if (pc == 0) SPMV3(0, 0); else if (pc == 1) SPMV3(0, 1); else SPMV3(0, 2);
     } else {
@@ -698,13 +698,13 @@ static int spmv32_pc(cfdgpu_handle *h, const float *x, float *y, const GmresStat
     else
       bsr4_spmv_f32<2><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, h->dinv32, h->binv32, y, st, j, xscale, active);
   } else {
-    const int grid = (int)((h->n + 255) / 256);
+    const int grid = (int)((h->nNode * 32LL + 255) / 256);
     if (pc == 0)
-      bsr_spmv_generic_f32<3, 0><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, h->dinv32, h->binv32, y, st, j, xscale, active);
+      bsr3_spmv<0, 0, float, float><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, y, st, j, xscale, active);
     else if (pc == 1)
-      bsr_spmv_generic_f32<3, 1><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, h->dinv32, h->binv32, y, st, j, xscale, active);
+      bsr3_spmv<0, 1, float, float><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, y, st, j, xscale, active);
     else
-      bsr_spmv_generic_f32<3, 2><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, h->dinv32, h->binv32, y, st, j, xscale, active);
+      bsr3_spmv<0, 2, float, float><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, y, st, j, xscale, active);
   }
   prof_end(h, pi);
   LAUNCHED(h);
@@ -771,14 +771,17 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
   const int64_t ldv = K.ldv;
   const int64_t nchunk = ldv / E;
   const int ntiles = (int)((nchunk + ORTHO_THREADS - 1) / ORTHO_THREADS);
-  const int mtiles = (int)(nchunk / MAXPY_SPAN);
+  // a flexible cycle keeps to the tiled forms: it has few vectors, and its FP32
+  // inner solves carry any other order of these sums on into the result
+  const bool few = nchunk <= MAXPY_FEW && !K.Z, each = nchunk <= MDOT_EACH && !K.Z;
+  const int mtiles = maxpy_tiles(nchunk, few);
   VT *V = K.V;
   GmresState *st = K.st;
   int rc;
   gmres_init<<<1, 1, 0, h->stream>>>(st, m, max_it, rtol, atol, dtol);
   LAUNCHED(h);
   CK(cudaMemsetAsync(x, 0, sizeof(double) * n, h->stream));
-  const int vgrid = grid_for(n);
+  const int ugrid = (int)std::min<int64_t>((n + UPDATE_SPAN - 1) / UPDATE_SPAN, 8 * 148);
   // Arnoldi steps j0..j0+CH-1 enqueued as one unit: directly, or (without
   // per-kernel profiling) as a CUDA graph captured once per chunk and reused
   const int CH = h->chunk;
@@ -787,9 +790,16 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
       int r;
       if ((r = arnoldi(j))) return r;
       const int pi = prof_begin(h, CFDGPU_KIND_ORTHO, (2.0 * j + 3.0) * (double)sizeof(VT) * n);
-      dim3 g2(ntiles, (j + 1 + MDOT_KC - 1) / MDOT_KC);
-      gmres_mdot<VT><<<g2, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
-      gmres_maxpy_norm<VT><<<mtiles, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      if (each) {
+        gmres_mdot_each<VT><<<j + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      } else {
+        dim3 g2(ntiles, (j + 1 + MDOT_KC - 1) / MDOT_KC);
+        gmres_mdot<VT><<<g2, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      }
+      if (few)
+        gmres_maxpy_norm<VT, MAXPY_FEW_SPAN, 1, 8><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      else
+        gmres_maxpy_norm<VT, MAXPY_WIDE_SPAN / 2, 2, 2><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
       prof_end(h, pi);
     }
     return check_launch(h, "gmres_arnoldi");
@@ -841,12 +851,12 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
         if (!h->h_gst[pidx].active) stop = true;
       }
     }
-    gmres_backsub<<<1, 1024, 0, h->stream>>>(st, K.ga);
+    gmres_backsub<<<1, BACKSUB_THREADS, 0, h->stream>>>(st, K.ga);
     h->launches += 1;
     if (K.Z)
-      gmres_update_x<double><<<vgrid, ORTHO_THREADS, 0, h->stream>>>(n, x, K.Z, ldv, st, K.gaz, 1.0);
+      gmres_update_x<double><<<ugrid, ORTHO_THREADS, 0, h->stream>>>(n, x, K.Z, ldv, st, K.gaz, 1.0);
     else
-      gmres_update_x<VT><<<vgrid, ORTHO_THREADS, 0, h->stream>>>(n, x, V, ldv, st, K.ga, 1.0);
+      gmres_update_x<VT><<<ugrid, ORTHO_THREADS, 0, h->stream>>>(n, x, V, ldv, st, K.ga, 1.0);
     h->launches += 1;
     if ((rc = check_launch(h, "gmres_build_soln"))) return rc;
     GmresState *fin = h->h_gst + cfdgpu_handle::MAX_DEPTH + 1;
@@ -1304,8 +1314,9 @@ int cfdgpu_create(const cfdgpu_mesh *mesh, const cfdgpu_control *ctrl, const cfd
   if ((rc = dalloc(h, &h->ga.grs, (size_t)h->m + 1))) return rc;
   if ((rc = dalloc(h, &h->ga.y, (size_t)h->m))) return rc;
   {
-    const int64_t ntiles = (h->ldv / 2 + ORTHO_THREADS - 1) / ORTHO_THREADS + h->ldv / 2 / MAXPY_SPAN + 1;
-    if ((rc = dalloc(h, &h->ga.partial, (size_t)(h->m + 1) * std::max<int64_t>(ntiles, RED_BLOCKS)))) return rc;
+    // (m + 1) rows of the multi-dot's tiles, or the tiles of the update
+    const int64_t ntiles = std::max<int64_t>((h->ldv / 2 + ORTHO_THREADS - 1) / ORTHO_THREADS, RED_BLOCKS);
+    if ((rc = dalloc(h, &h->ga.partial, (size_t)std::max<int64_t>((h->m + 1) * ntiles, maxpy_tiles(h->ldv / 2, h->ldv / 2 <= MAXPY_FEW))))) return rc;
   }
   if ((rc = dalloc(h, &h->ga.coef, (size_t)h->m + 1))) return rc;
   if ((rc = dalloc(h, &h->ga.kcount, (size_t)h->m / MDOT_KC + 2))) return rc;
@@ -1989,9 +2000,9 @@ extern "C" int cfdgpu_residual_norm_noalloc(int nNode, int ndof, const int32_t *
     bsr4_spmv<1, 0, double><<<grid, 256, 0, s>>>(nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr, r,
                                                 nullptr, 0, nullptr);
   } else {
-    const int grid = (int)((n + 255) / 256);
-    bsr_spmv_generic<3, 1, 0, double><<<grid, 256, 0, s>>>(nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr,
-                                                             nullptr, r, nullptr, 0, nullptr);
+    const int grid = (int)((nNode * 32LL + 255) / 256);
+    bsr3_spmv<1, 0, double, double><<<grid, 256, 0, s>>>(nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr,
+                                                         r, nullptr, 0, nullptr);
   }
   if (cudaGetLastError() != cudaSuccess) return CFDGPU_ECUDA;
   norm2_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, r, partial, counter, d_norm);

@@ -210,98 +210,72 @@ bsr4_spmv_f32(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__re
   }
 }
 
-// Generic BSR SpMV for any block size NB (used for 3x3 blocks): one thread
-// per scalar row.
-template <int NB, int MODE, int PC, typename VT>
-__global__ void bsr_spmv_generic(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                 const VT *__restrict__ val, const double *__restrict__ x, const double *__restrict__ b,
-                                 const double *__restrict__ dinv, const double *__restrict__ binv,
-                                 double *__restrict__ y, const GmresState *__restrict__ st, int j,
-                                 const double *__restrict__ xscale, const int *__restrict__ active = nullptr)
+// BSR SpMV, 3x3 blocks (2D): one warp per block row.  Lanes 3*sub + row load row
+// 'row' of block 'sub' of ten and entry 'row' of its x, so the nine blocks of a
+// quadrilateral mesh's row are one pass of contiguous loads; lanes 0, 1 and 2 then
+// add a row each from shared memory, entry after entry.  Bound by the chain row
+// pointer -> column -> x -> sum (27 FMAs); the preconditioner's entries are loaded
+// ahead of it.  One thread per scalar row with the same sums, which waited for its
+// blocks one after another and with point-block Jacobi went over the whole node
+// three times, took 5.7 us (Jacobi, 363 unknowns) and 7.9 (point-block, 10,092);
+// now 2.4 and 3.6.  ST: type of the vectors and of the sums; MT: of the blocks.
+template <int MODE, int PC, typename MT, typename ST>
+__global__ void __launch_bounds__(256)
+bsr3_spmv(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
+          const MT *__restrict__ val, const ST *__restrict__ x, const ST *__restrict__ b,
+          const ST *__restrict__ dinv, const ST *__restrict__ binv, ST *__restrict__ y,
+          const GmresState *__restrict__ st, int j, const double *__restrict__ xscale,
+          const int *__restrict__ active = nullptr)
 {
   if (st && (!st->active || st->it != j)) return;
   if (active && !active[0]) return;
-  const double xs = xscale ? xscale[0] : 1.0;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t node = t / NB;
-  const int row = (int)(t % NB);
+  constexpr int PASS = 10;                       // blocks per pass; a row of 30 entries keeps 16-byte pairs
+  __shared__ __align__(16) ST sa[8][3][3 * PASS], sx[8][3 * PASS];
+  const int w = threadIdx.x >> 5, node = blockIdx.x * 8 + w;
+  const int lane = threadIdx.x & 31;
   if (node >= nrows) return;
-  double acc = 0.0;
-  for (int kb = rowptr[node]; kb < rowptr[node + 1]; kb++) {
-    const int c = colidx[kb];
-    const VT *a = val + (int64_t)kb * NB * NB + row * NB;
-#pragma unroll
-    for (int q = 0; q < NB; q++) acc = fma((double)a[q], x[(int64_t)c * NB + q], acc);
-  }
-  double v = (MODE == 1) ? b[t] - xs * acc : xs * acc;
-  if (PC == 1) v *= dinv[t];
-  if (PC == 2) {
-    // point block needs the whole node: recompute the node's other rows
-    double vv[NB];
-#pragma unroll
-    for (int rr = 0; rr < NB; rr++) {
-      double s = 0.0;
-      for (int kb = rowptr[node]; kb < rowptr[node + 1]; kb++) {
-        const int c = colidx[kb];
-        const VT *a = val + (int64_t)kb * NB * NB + rr * NB;
-#pragma unroll
-        for (int q = 0; q < NB; q++) s = fma((double)a[q], x[(int64_t)c * NB + q], s);
-      }
-      vv[rr] = (MODE == 1) ? b[node * NB + rr] - xs * s : xs * s;
-    }
-    double z = 0.0;
-#pragma unroll
-    for (int q = 0; q < NB; q++) z += binv[node * NB * NB + row * NB + q] * vv[q];
-    v = z;
-  }
-  y[t] = v;
-}
-
-// The same for other block sizes (3x3 in 2D), FP32 blocks and vectors: one
-// thread per scalar row, FP32 accumulation as in the 4x4 FP32 kernel.
-template <int NB, int PC>
-__global__ void bsr_spmv_generic_f32(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                                     const float *__restrict__ val, const float *__restrict__ x,
-                                     const float *__restrict__ dinv, const float *__restrict__ binv,
-                                     float *__restrict__ y, const GmresState *__restrict__ st, int j,
-                                     const double *__restrict__ xscale, const int *__restrict__ active = nullptr)
-{
-  if (st && (!st->active || st->it != j)) return;
-  if (active && !active[0]) return;
-  const float xs = xscale ? (float)xscale[0] : 1.f;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t node = t / NB;
-  const int row = (int)(t % NB);
-  if (node >= nrows) return;
+  const ST xs = xscale ? (ST)xscale[0] : (ST)1;
+  const int sub = lane / 3, row = lane - 3 * sub;
   const int kb0 = rowptr[node], kb1 = rowptr[node + 1];
-  if (PC == 2) {
-    float vv[NB];
+  const int64_t r = (int64_t)node * 3 + row;
+  ST pc[3] = {}, br = 0;
+  if (lane < 3) {
+    if (MODE == 1) br = b[r];
+    if (PC == 1) pc[0] = dinv[r];
+    if (PC == 2) {
 #pragma unroll
-    for (int rr = 0; rr < NB; rr++) {
-      float s = 0.f;
-      for (int kb = kb0; kb < kb1; kb++) {
-        const int c = colidx[kb];
-        const float *a = val + (int64_t)kb * NB * NB + rr * NB;
-#pragma unroll
-        for (int q = 0; q < NB; q++) s = fmaf(a[q], x[(int64_t)c * NB + q], s);
-      }
-      vv[rr] = xs * s;
+      for (int q = 0; q < 3; q++) pc[q] = binv[r * 3 + q];
     }
-    float z = 0.f;
-#pragma unroll
-    for (int q = 0; q < NB; q++) z += binv[node * NB * NB + row * NB + q] * vv[q];
-    y[t] = z;
-    return;
   }
-  float acc = 0.f;
-  for (int kb = kb0; kb < kb1; kb++) {
-    const int c = colidx[kb];
-    const float *a = val + (int64_t)kb * NB * NB + row * NB;
+  ST acc = 0;
+  for (int k0 = kb0; k0 < kb1; k0 += PASS) {
+    const int kb = k0 + sub;
+    if (sub < PASS) {
+      ST a[3] = {}, xv = 0;
+      if (kb < kb1) {
+        xv = x[(int64_t)colidx[kb] * 3 + row];
 #pragma unroll
-    for (int q = 0; q < NB; q++) acc = fmaf(a[q], x[(int64_t)c * NB + q], acc);
+        for (int q = 0; q < 3; q++) a[q] = (ST)val[(int64_t)kb * 9 + row * 3 + q];
+      }
+#pragma unroll
+      for (int q = 0; q < 3; q++) sa[w][row][3 * sub + q] = a[q];
+      sx[w][3 * sub + row] = xv;
+    }
+    __syncwarp();
+    if (lane < 3) {
+#pragma unroll
+      for (int k = 0; k < 3 * PASS; k++) acc = fma(sa[w][row][k], sx[w][k], acc);
+    }
+    __syncwarp();
   }
-  acc *= xs;
-  y[t] = (PC == 1) ? dinv[t] * acc : acc;
+  ST v = (MODE == 1) ? br - xs * acc : xs * acc;
+  if (PC == 1) v *= pc[0];
+  if (PC == 2) {
+    const ST v0 = __shfl_sync(0xffffffffu, v, 0), v1 = __shfl_sync(0xffffffffu, v, 1);
+    const ST v2 = __shfl_sync(0xffffffffu, v, 2);
+    v = fma(pc[2], v2, fma(pc[1], v1, pc[0] * v0));
+  }
+  if (lane < 3) y[r] = v;
 }
 
 // z = M^-1 r (stand-alone preconditioner application)
@@ -378,6 +352,32 @@ __global__ void build_jacobi(int nnode, const int32_t *__restrict__ diag_slot, c
     for (int c = 0; c < NB; c++) binv[(int64_t)node * NB * NB + a * NB + c] = (PT)I[a][c];
 }
 
+// The last CTA's sum of a grid's partials, all threads loading (fixed tree);
+// result valid in thread 0.
+__device__ __forceinline__ double sum_partials(const double *partial, unsigned int count, double *sh)
+{
+  double t = 0.0;
+  for (unsigned int k = threadIdx.x; k < count; k += RED_THREADS) t += __ldcg(partial + k);
+  return block_sum<RED_THREADS>(t, sh);
+}
+
+// The same one after another, result valid in thread 0; count <= RED_BLOCKS.  One
+// thread that also loaded the 296 partials was most of the 11 us that a norm took.
+__device__ __forceinline__ double sum_partials_in_order(const double *partial, unsigned int count)
+{
+  __shared__ double all[RED_BLOCKS];
+  for (unsigned int k = threadIdx.x; k < count; k += RED_THREADS) all[k] = __ldcg(partial + k);
+  __syncthreads();
+  return threadIdx.x == 0 ? sum_in_order(all, count) : 0.0;
+}
+
+// CTAs of a reduction over n entries: four entries per thread, at most RED_BLOCKS
+inline int red_grid(int64_t n)
+{
+  const int64_t g = (n + 4 * RED_THREADS - 1) / (4 * RED_THREADS);
+  return (int)(g < 1 ? 1 : g > RED_BLOCKS ? RED_BLOCKS : g);
+}
+
 // ---------------------------------------------------------------------------
 // deterministic 2-norm: out[0] = ||x||; partials in scratch
 __global__ void __launch_bounds__(RED_THREADS)
@@ -391,11 +391,8 @@ norm2_kernel(int64_t n, const double *__restrict__ x, double *__restrict__ parti
   s = block_sum<RED_THREADS>(s, sh);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
   if (last_block(counter, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) t += __ldcg(partial + k);
-      out[0] = sqrt(t);
-    }
+    const double t = sum_partials_in_order(partial, gridDim.x);
+    if (threadIdx.x == 0) out[0] = sqrt(t);
   }
 }
 
@@ -427,32 +424,6 @@ template <> struct Chunk<float> {
   }
 };
 
-// out[0] = <a, a - b>, out[1] = ||a - b||^2 (deterministic; partial holds
-// 2 * gridDim.x doubles)
-__global__ void __launch_bounds__(RED_THREADS)
-minres_dots(int64_t n, const double *__restrict__ a, const double *__restrict__ b, double *__restrict__ partial,
-            unsigned int *counter, double *__restrict__ out)
-{
-  __shared__ double sh[RED_THREADS / 32];
-  double s0 = 0.0, s1 = 0.0;
-  for (int64_t i = (int64_t)blockIdx.x * RED_THREADS + threadIdx.x; i < n; i += (int64_t)gridDim.x * RED_THREADS) {
-    const double d = a[i] - b[i];
-    s0 = fma(a[i], d, s0);
-    s1 = fma(d, d, s1);
-  }
-  s0 = block_sum<RED_THREADS>(s0, sh);
-  s1 = block_sum<RED_THREADS>(s1, sh);
-  if (threadIdx.x == 0) { partial[2 * blockIdx.x] = s0; partial[2 * blockIdx.x + 1] = s1; }
-  if (last_block(counter, gridDim.x)) {
-    if (threadIdx.x == 0) {
-      double t0 = 0.0, t1 = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) { t0 += __ldcg(partial + 2 * k); t1 += __ldcg(partial + 2 * k + 1); }
-      out[0] = t0;
-      out[1] = t1;
-    }
-  }
-}
-
 // Gram data of two residual differences k_i = a - b_i (deterministic):
 // out = [<a,k1>, <a,k2>, <k1,k1>, <k1,k2>, <k2,k2>]; partial holds 5*gridDim.x
 __global__ void __launch_bounds__(RED_THREADS)
@@ -475,11 +446,10 @@ minres_dots2(int64_t n, const double *__restrict__ a, const double *__restrict__
     if (threadIdx.x == 0) partial[5 * blockIdx.x + q] = t;
   }
   if (last_block(counter, gridDim.x)) {
-    if (threadIdx.x < 5) {
-      double t = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) t += __ldcg(partial + 5 * k + threadIdx.x);
-      out[threadIdx.x] = t;
-    }
+    __shared__ double all[5][RED_BLOCKS];
+    for (unsigned int k = threadIdx.x; k < 5 * gridDim.x; k += RED_THREADS) all[k % 5][k / 5] = __ldcg(partial + k);
+    __syncthreads();
+    if (threadIdx.x < 5) out[threadIdx.x] = sum_in_order(all[threadIdx.x], gridDim.x);
   }
 }
 
@@ -497,9 +467,8 @@ gmres_start(int64_t n, const VT *__restrict__ v0, GmresState *st, GmresArrays ga
   s = block_sum<RED_THREADS>(s, sh);
   if (threadIdx.x == 0) ga.partial[blockIdx.x] = s;
   if (last_block(&st->counter, gridDim.x)) {
+    const double t = sum_partials_in_order(ga.partial, gridDim.x);
     if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (unsigned int k = 0; k < gridDim.x; k++) t += __ldcg(ga.partial + k);
       const double res = sqrt(t);
       st->res = res;
       st->it = 0;
@@ -596,92 +565,161 @@ gmres_mdot(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, const G
   }
 }
 
-// w -= sum_k h_k sigma_k V_k, then ||w||^2 partials.  A CTA covers
-// 2*MAXPY_CHUNKS 16-byte chunks: each thread owns two chunks (lp and
-// lp + MAXPY_CHUNKS, two independent load streams), its quarter of the CTA
-// takes the k's congruent to 0..3 mod 4 (consecutive lanes on consecutive
-// chunks), and the quarter sums are combined in a fixed order through shared
-// memory.  The last CTA finishes the norm, applies the stored Givens rotations
-// to column j, forms the new one and runs the convergence test
-// (KSPGMRESUpdateHessenberg, KSPConvergedDefault).
-constexpr int MAXPY_CHUNKS = 64;
-constexpr int MAXPY_SPAN = 2 * MAXPY_CHUNKS;   // chunks per CTA
+// The same for few unknowns: one CTA per basis vector, which needs no second
+// stage over partial sums (a fence, an atomic and a dependent read, a third of
+// the multi-dot's 3.7 us at 363 unknowns; now 1.9).  Up to MDOT_EACH chunks, eight loads
+// per thread; beyond, w would be read from L2 once for every vector.
+constexpr int64_t MDOT_EACH = 8 * ORTHO_THREADS;
 template <typename VT>
 __global__ void __launch_bounds__(ORTHO_THREADS)
-gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresState *st, GmresArrays ga)
+gmres_mdot_each(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, const GmresState *__restrict__ st,
+                GmresArrays ga)
 {
   if (!st->active || st->it != j) return;
   constexpr int E = Chunk<VT>::E;
   __shared__ double sh[ORTHO_THREADS / 32];
-  __shared__ double qs[ORTHO_THREADS / MAXPY_CHUNKS][E][MAXPY_SPAN];
+  const int k = blockIdx.x;
+  const VT *v = V + (int64_t)k * ldv, *w = V + (int64_t)(j + 1) * ldv;
+  const double sigma = ga.sigma[k];
+  double acc = 0.0;
+#pragma unroll 4
+  for (int64_t p = threadIdx.x; p < nchunk; p += ORTHO_THREADS) {
+    double a[E], b[E];
+    Chunk<VT>::load(v + E * p, a);
+    Chunk<VT>::load(w + E * p, b);
+#pragma unroll
+    for (int e = 0; e < E; e++) acc = fma(a[e], b[e], acc);
+  }
+  acc = block_sum<ORTHO_THREADS>(acc, sh);
+  if (threadIdx.x == 0) {
+    const double hkj = sigma * acc;
+    ga.H[hidx(k, j, st->m)] = hkj;
+    ga.coef[k] = hkj * sigma;
+  }
+}
+
+// w -= sum_k h_k sigma_k V_k, then ||w||^2 partials.  A CTA covers CL * PER
+// 16-byte chunks; its threads are 256 / CL groups of CL: group g adds the k's
+// congruent to g modulo the number of groups, each thread for its PER chunks,
+// UN terms in flight, and the groups' sums are combined in a fixed order
+// through shared memory.  One more CTA applies the stored Givens rotations to
+// column j meanwhile (a serial chain of j steps, none of which needs the norm);
+// the last CTA to arrive finishes the norm, forms the new rotation and runs the
+// convergence test (KSPGMRESUpdateHessenberg, KSPConvergedDefault).
+//
+// Many unknowns (64 x 2 chunks): bound by reading V, 2 KB of a vector per CTA.  Few
+// unknowns (16 x 1): V comes from L2 and the time is the latency of the terms that a
+// thread adds one batch after another, so each CTA takes 16 chunks with 16
+// groups, which fills the SMs and cuts the chain to j / 128 batches.
+// With the wide form for every size and the rotations after the norm: 6.5 us at 363
+// unknowns and 50 vectors, 15.5 at 10,092 and 300; now 4.8 and 8.4.
+constexpr int MAXPY_FEW_SPAN = 16, MAXPY_WIDE_SPAN = 128;
+// up to eight CTAs an SM in the narrow form (38,000 FP64 unknowns)
+constexpr int64_t MAXPY_FEW = (int64_t)MAXPY_FEW_SPAN * 8 * 148;
+inline int maxpy_tiles(int64_t nchunk, bool few)
+{
+  const int span = few ? MAXPY_FEW_SPAN : MAXPY_WIDE_SPAN;
+  return (int)((nchunk + span - 1) / span);
+}
+template <typename VT, int CL, int PER, int UN>
+__global__ void __launch_bounds__(ORTHO_THREADS, PER > 1 ? 5 : 3)
+gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresState *st, GmresArrays ga)
+{
+  if (!st->active || st->it != j) return;
+  constexpr int E = Chunk<VT>::E, SPAN = CL * PER, GROUPS = ORTHO_THREADS / CL;
+  static_assert(SPAN <= ORTHO_THREADS, "");
+  __shared__ double sh[ORTHO_THREADS / 32];
+  __shared__ union {
+    double qs[GROUPS][E][SPAN];
+    double col[3][1024];           // column j, cosines, sines of the rotation CTA
+  } u;
   const int m = st->m;
-  // coefficients H(k, j) sigma_k (written by the multi-dot), read as
-  // warp-uniform broadcasts inside the loop
-  const double *__restrict__ hk = ga.coef;
-  VT *w = V + (int64_t)(j + 1) * ldv;
-  const int lp = threadIdx.x % MAXPY_CHUNKS;
-  const int quarter = threadIdx.x / MAXPY_CHUNKS;
-  const int64_t p0 = (int64_t)blockIdx.x * MAXPY_SPAN + lp;
-  const int64_t p1 = p0 + MAXPY_CHUNKS;
-  // the chunk of w this thread finishes (quarters 0 and 1), loaded early
-  const int cfin = lp + (quarter & 1) * MAXPY_CHUNKS;
-  const int64_t pfin = (int64_t)blockIdx.x * MAXPY_SPAN + cfin;
-  double wfin[E];
-  if (quarter < 2 && pfin < nchunk) Chunk<VT>::load(w + E * pfin, wfin);
-  double a0[E], a1[E];
+  const int tiles = (int)gridDim.x - 1;
+  if ((int)blockIdx.x == tiles) {
+    double *hc = u.col[0], *rc = u.col[1], *rs = u.col[2];
+    double *Hj = ga.H + hidx(0, j, m);
+    for (int q = threadIdx.x; q <= j; q += ORTHO_THREADS) {
+      hc[q] = Hj[q];
+      if (q < j) { rc[q] = ga.cs[q]; rs[q] = ga.sn[q]; }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double a = hc[0];
+#pragma unroll 8
+      for (int q = 0; q < j; q++) {
+        const double c = rc[q], sn = rs[q], bq = hc[q + 1];
+        rc[q] = c * a + sn * bq;   // the rotated entry q
+        a = c * bq - sn * a;
+      }
+      rc[j] = a;
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q <= j; q += ORTHO_THREADS) Hj[q] = rc[q];
+  } else {
+    // coefficients H(k, j) sigma_k (written by the multi-dot), read as
+    // group-uniform broadcasts inside the loop
+    const double *__restrict__ hk = ga.coef;
+    VT *w = V + (int64_t)(j + 1) * ldv;
+    const int lp = threadIdx.x % CL, g = threadIdx.x / CL;
+    const int64_t c0 = (int64_t)blockIdx.x * SPAN;
+    // the chunk of w this thread finishes, loaded early; nchunk is a multiple
+    // of 16 (ldv is one of 32 entries), the spans may reach past it
+    const int64_t pfin = c0 + threadIdx.x;
+    const bool fin = threadIdx.x < SPAN && pfin < nchunk;
+    double wfin[E];
+    if (fin) Chunk<VT>::load(w + E * pfin, wfin);
+    double acc[PER][E] = {};
+    const VT *bp[PER];
+    bool in[PER];
 #pragma unroll
-  for (int e = 0; e < E; e++) { a0[e] = 0.0; a1[e] = 0.0; }
-  // nchunk is a multiple of 16 (ldv is a multiple of 32 entries), so a CTA
-  // either owns both chunks of a thread or neither past the end
-  if (p1 < nchunk) {
-    const VT *b0 = V + E * p0;
-    const VT *b1 = V + E * p1;
-    int k = quarter;
-    for (; k + 4 <= j; k += 8) {
-      double v0[E], v1[E], u0[E], u1[E];
-      const double c0 = __ldg(hk + k), c1 = __ldg(hk + k + 4);
-      Chunk<VT>::load(b0 + (int64_t)k * ldv, v0);
-      Chunk<VT>::load(b1 + (int64_t)k * ldv, u0);
-      Chunk<VT>::load(b0 + (int64_t)(k + 4) * ldv, v1);
-      Chunk<VT>::load(b1 + (int64_t)(k + 4) * ldv, u1);
+    for (int i = 0; i < PER; i++) {
+      const int64_t p = c0 + lp + i * CL;
+      in[i] = p < nchunk;
+      bp[i] = V + E * (in[i] ? p : c0);
+    }
+    if (in[0]) {
+      for (int k = g; k <= j; k += GROUPS * UN) {
+        double v[UN][PER][E], c[UN];
 #pragma unroll
-      for (int e = 0; e < E; e++) {
-        a0[e] = fma(c0, v0[e], a0[e]);
-        a1[e] = fma(c0, u0[e], a1[e]);
-        a0[e] = fma(c1, v1[e], a0[e]);
-        a1[e] = fma(c1, u1[e], a1[e]);
+        for (int t = 0; t < UN; t++) {
+          const int kt = k + t * GROUPS;
+          if (kt <= j) {
+            c[t] = __ldg(hk + kt);
+#pragma unroll
+            for (int i = 0; i < PER; i++) Chunk<VT>::load(bp[i] + (int64_t)kt * ldv, v[t][i]);
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < UN; t++) {
+          if (k + t * GROUPS <= j) {
+#pragma unroll
+            for (int i = 0; i < PER; i++)
+#pragma unroll
+              for (int e = 0; e < E; e++) acc[i][e] = fma(c[t], v[t][i][e], acc[i][e]);
+          }
+        }
       }
     }
-    for (; k <= j; k += 4) {
-      double v0[E], u0[E];
-      const double c0 = __ldg(hk + k);
-      Chunk<VT>::load(b0 + (int64_t)k * ldv, v0);
-      Chunk<VT>::load(b1 + (int64_t)k * ldv, u0);
 #pragma unroll
-      for (int e = 0; e < E; e++) {
-        a0[e] = fma(c0, v0[e], a0[e]);
-        a1[e] = fma(c0, u0[e], a1[e]);
-      }
-    }
-  }
+    for (int i = 0; i < PER; i++)
 #pragma unroll
-  for (int e = 0; e < E; e++) {
-    qs[quarter][e][lp] = a0[e];
-    qs[quarter][e][lp + MAXPY_CHUNKS] = a1[e];
-  }
-  __syncthreads();
-  double s = 0.0;
-  // quarter q < 2 finishes chunk lp + q*MAXPY_CHUNKS
-  if (quarter < 2) {
-    const int c = cfin;
-    const int64_t p = pfin;
-    if (p < nchunk) {
+      for (int e = 0; e < E; e++) u.qs[g][e][lp + i * CL] = acc[i][e];
+    __syncthreads();
+    double s = 0.0;
+    if (fin) {
       double a[E];
 #pragma unroll
-      for (int e = 0; e < E; e++) a[e] = wfin[e];
+      for (int e = 0; e < E; e++) {
+        double q[GROUPS];
 #pragma unroll
-      for (int e = 0; e < E; e++) a[e] -= ((qs[0][e][c] + qs[1][e][c]) + (qs[2][e][c] + qs[3][e][c]));
-      Chunk<VT>::store(w + E * p, a);
+        for (int i = 0; i < GROUPS; i++) q[i] = u.qs[i][e][threadIdx.x];
+#pragma unroll
+        for (int d = 1; d < GROUPS; d *= 2)
+#pragma unroll
+          for (int i = 0; i < GROUPS; i += 2 * d) q[i] += q[i + d];
+        a[e] = wfin[e] - q[0];
+      }
+      Chunk<VT>::store(w + E * pfin, a);
       // the norm is taken of the stored (possibly rounded) values
 #pragma unroll
       for (int e = 0; e < E; e++) {
@@ -689,53 +727,37 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
         s = fma(v, v, s);
       }
     }
+    s = block_sum<ORTHO_THREADS>(s, sh);
+    if (threadIdx.x == 0) ga.partial[blockIdx.x] = s;
   }
-  s = block_sum<ORTHO_THREADS>(s, sh);
-  if (threadIdx.x == 0) ga.partial[blockIdx.x] = s;
   if (last_block(&st->counter, gridDim.x)) {
-    double t = 0.0;
-    for (unsigned int b = threadIdx.x; b < gridDim.x; b += ORTHO_THREADS) t += __ldcg(ga.partial + b);
-    t = block_sum<ORTHO_THREADS>(t, sh);
-    // stage column j of H and the stored rotations in shared memory (hk is
-    // free again), so the serial rotation chain below runs from registers and
-    // shared memory instead of global-memory round trips
-    __shared__ double rc[1024], rs[1024], hc[1024];
-    const int it = j;
-    for (int q = threadIdx.x; q <= it; q += blockDim.x) hc[q] = ga.H[hidx(q, it, m)];
-    for (int q = threadIdx.x; q < it; q += blockDim.x) { rc[q] = ga.cs[q]; rs[q] = ga.sn[q]; }
-    __syncthreads();
+    double a = 0.0, g0 = 0.0;
+    if (threadIdx.x == 0) { a = __ldcg(ga.H + hidx(j, j, m)); g0 = __ldcg(ga.grs + j); }
+    const double t = sum_partials(ga.partial, tiles, sh);
     if (threadIdx.x == 0) {
+      const int it = j;
       const double tt = sqrt(t);
       st->tt = tt;
       ga.sigma[it + 1] = (tt != 0.0) ? 1.0 / tt : 1.0;   // VecNormalize, applied lazily
-      hc[it + 1] = tt;
-      double hapbnd = fabs(tt / ga.grs[it]);
+      double hapbnd = fabs(tt / g0);
       if (hapbnd > 1.0e-30) hapbnd = 1.0e-30;
       const bool hapend = tt < hapbnd;
-      // apply the previous rotations to the new column
-      double a = hc[0];
-      for (int q = 1; q <= it; q++) {
-        const double bq = hc[q];
-        hc[q - 1] = rc[q - 1] * a + rs[q - 1] * bq;
-        a = rc[q - 1] * bq - rs[q - 1] * a;
-      }
-      hc[it] = a;
       double res;
       int reason = 0;
       if (!hapend) {
-        const double bq = hc[it + 1];
-        const double r = sqrt(a * a + bq * bq);
+        const double r = sqrt(a * a + tt * tt);
         if (r == 0.0) {
           reason = -2;   // KSP_DIVERGED_NULL
           res = st->res;
         } else {
-          const double c = a / r, sn = bq / r;
+          const double c = a / r, sn = tt / r;
           ga.cs[it] = c;
           ga.sn[it] = sn;
-          ga.grs[it + 1] = -(sn * ga.grs[it]);
-          ga.grs[it] = c * ga.grs[it];
-          hc[it] = c * a + sn * bq;
-          res = fabs(ga.grs[it + 1]);
+          res = -(sn * g0);
+          ga.grs[it + 1] = res;
+          ga.grs[it] = c * g0;
+          ga.H[hidx(it, it, m)] = c * a + sn * tt;
+          res = fabs(res);
         }
       } else {
         res = 0.0;
@@ -750,50 +772,104 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
       st->reason = reason;
       st->active = (reason == 0 && st->it < m && st->its < st->maxit) ? 1 : 0;
     }
-    __syncthreads();
-    for (int q = threadIdx.x; q <= it + 1; q += blockDim.x) ga.H[hidx(q, it, m)] = hc[q];
   }
 }
 
-// KSPGMRESBuildSoln back substitution, column-oriented: one CTA; for k from
-// the last column down, y_k = r_k / H(k,k), then r_i -= H(i,k) y_k for i < k.
-__global__ void __launch_bounds__(1024) gmres_backsub(GmresState *st, GmresArrays ga)
+// KSPGMRESBuildSoln back substitution, one CTA, 32 columns at a time from the
+// last: one warp solves the diagonal block from registers (lane i holds row i,
+// each y travels by shuffle), then the rows above take the block's columns, a
+// thread each.  A quotient is r * (1/d) with one correction
+// step, so the division is off the chain and the result as good as r / d.
+// Bound by that chain, 60 cycles a column; a column at a time over the whole CTA,
+// with a load, a division and two barriers in turn, took 280 us for 290 columns; now 45.
+constexpr int BACKSUB_THREADS = 256;
+__global__ void __launch_bounds__(BACKSUB_THREADS) gmres_backsub(GmresState *st, GmresArrays ga)
 {
   __shared__ double r[1024];
-  __shared__ double yk;
-  const int last = st->it - 1;
-  const int m = st->m;
-  if (last < 0) return;
-  for (int i = threadIdx.x; i <= last; i += blockDim.x) r[i] = ga.grs[i];
-  __syncthreads();
-  for (int k = last; k >= 0; k--) {
-    if (threadIdx.x == 0) {
-      const double d = ga.H[hidx(k, k, m)];
-      yk = (d != 0.0) ? r[k] / d : 0.0;
-      ga.y[k] = yk;
+  __shared__ double ys[32];
+  const int it = st->it, m = st->m;
+  if (it <= 0) return;
+  for (int i = threadIdx.x; i < it; i += BACKSUB_THREADS) r[i] = ga.grs[i];
+  const int lane = threadIdx.x & 31;
+  for (int k1 = it; k1 > 0;) {
+    const int k0 = (k1 - 1) & ~31, nc = k1 - k0;
+    double col[32], inv = 0.0, d = 0.0;
+    if (threadIdx.x < 32) {
+#pragma unroll
+      for (int c = 0; c < 32; c++) col[c] = (c < nc && lane < c) ? ga.H[hidx(k0 + lane, k0 + c, m)] : 0.0;
+      if (lane < nc) d = ga.H[hidx(k0 + lane, k0 + lane, m)];
+      inv = (d != 0.0) ? 1.0 / d : 0.0;
     }
     __syncthreads();
-    const double y = yk;
-    for (int i = threadIdx.x; i < k; i += blockDim.x) r[i] -= ga.H[hidx(i, k, m)] * y;
+    if (threadIdx.x < 32) {
+      double v = (lane < nc) ? r[k0 + lane] : 0.0;
+#pragma unroll
+      for (int c = 31; c >= 0; c--) {
+        double q = v * inv;
+        q = isfinite(q) ? fma(fma(-q, d, v), inv, q) : v / d;
+        const double y = __shfl_sync(0xffffffffu, q, c);
+        if (lane < c) v = fma(-col[c], y, v);
+        else if (lane == c) v = y;
+      }
+      if (lane < nc) ga.y[k0 + lane] = v;
+      ys[lane] = (lane < nc) ? v : 0.0;
+    }
     __syncthreads();
+    // rows above the block, a thread each
+    for (int i = threadIdx.x; i < k0; i += BACKSUB_THREADS) {
+      double h[32], v = r[i];
+#pragma unroll
+      for (int c = 0; c < 32; c++) h[c] = (c < nc) ? ga.H[hidx(i, k0 + c, m)] : 0.0;
+#pragma unroll
+      for (int c = 31; c >= 0; c--) v = fma(-h[c], ys[c], v);
+      r[i] = v;
+    }
+    k1 = k0;
   }
 }
 
-// x += scale * sum_{k < it} y_k sigma_k V_k  (x is FP64 whatever the basis type)
+// x += scale * sum_{k < it} y_k sigma_k V_k  (x is FP64 whatever the basis
+// type).  Up to 16 vectors a thread adds its entry's terms alone; from there on a
+// CTA covers 32 entries, its eight warps taking the k's modulo 8 with eight loads
+// in flight, so the latency of V is paid it / 64 times and not it / 4 times.
+constexpr int UPDATE_SPAN = 32, UPDATE_ALONE = 16;
 template <typename VT>
 __global__ void __launch_bounds__(ORTHO_THREADS)
 gmres_update_x(int64_t n, double *__restrict__ x, const VT *__restrict__ V, int64_t ldv,
                const GmresState *__restrict__ st, GmresArrays ga, double scale)
 {
+  constexpr int W = ORTHO_THREADS / 32;
   __shared__ double yk[1024];
+  __shared__ double sh[W][UPDATE_SPAN];
   const int it = st->it;
   if (it <= 0) return;
   for (int k = threadIdx.x; k < it; k += blockDim.x) yk[k] = ga.y[k] * ga.sigma[k];
   __syncthreads();
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  if (it <= UPDATE_ALONE) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+      double s = 0.0;
+      for (int k = 0; k < it; k++) s = fma(yk[k], (double)V[(int64_t)k * ldv + i], s);
+      x[i] += scale * s;
+    }
+    return;
+  }
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t i0 = (int64_t)blockIdx.x * UPDATE_SPAN; i0 < n; i0 += (int64_t)gridDim.x * UPDATE_SPAN) {
+    const int64_t i = i0 + lane;
     double s = 0.0;
-    for (int k = 0; k < it; k++) s = fma(yk[k], (double)V[(int64_t)k * ldv + i], s);
-    x[i] += scale * s;
+    if (i < n) {
+#pragma unroll 8
+      for (int k = w; k < it; k += W) s = fma(yk[k], (double)V[(int64_t)k * ldv + i], s);
+    }
+    sh[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && i < n) {
+      double t = 0.0;
+#pragma unroll
+      for (int q = 0; q < W; q++) t += sh[q][lane];
+      x[i] += scale * t;
+    }
+    __syncthreads();
   }
 }
 
