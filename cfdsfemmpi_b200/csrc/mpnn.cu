@@ -215,48 +215,70 @@ __global__ void k_act(int64_t count, const float *__restrict__ z, const float *_
   }
 }
 
-// mean over the node's neighbourhood: out[i][c] = (1/deg_i) sum_j in[j][c]
-// (one warp per node, two channels per lane, neighbours in column order);
-// in/out strided (ld in elements); outb receives BF16, outf is accumulated
-// (FP32).  With transpose the inputs are divided by their own node's degree
-// instead (the transpose of the mean on the symmetric pattern).
-__global__ void k_mean_agg(int N, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
-                           const bf16 *__restrict__ in, int ldi, bf16 *__restrict__ outb, int ldo,
-                           const float *__restrict__ inf, float *__restrict__ outf, int transpose)
+// mean over the node's neighbourhood: out[i][c] = (1/deg_i) sum_j in[j][c],
+// neighbours in column order.  Half a warp per node, four channels per lane;
+// the 16 lanes load 16 column indices at once and hand them round, and the rows
+// of eight neighbours are in flight together.  T = bf16 input with leading
+// dimension ldi; the mean goes to outb as bf16 (leading dimension ldo).  TRANSPOSE
+// divides the inputs by their own node's degree instead (the transpose of the
+// mean on the symmetric pattern) and adds the sum to outf (FP32).
+// Bound by the rows' way from L2 and L1 (27 x 128 bytes a node on a hexahedral
+// mesh).  One load at a time after its own index took 202 us at
+// 274,625 nodes and 27 neighbours; now 144 (191 transposed).
+template <bool TRANSPOSE>
+__global__ void __launch_bounds__(256, 5)
+k_mean_agg(int N, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, const bf16 *__restrict__ in,
+           int ldi, bf16 *__restrict__ outb, int ldo, float *__restrict__ outf)
 {
-  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
+  constexpr int U = 8;
+  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
+  const int l = threadIdx.x & 15;
+  const int k0 = (node < N) ? rowptr[node] : 0, deg = (node < N) ? rowptr[node + 1] - k0 : 0;
+  const int other = __shfl_xor_sync(0xffffffffu, deg, 16);
+  const int most = max(deg, other);   // both halves of the warp take the same steps
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int base = 0; base < most; base += 16) {
+    int j = 0;
+    float sj = 1.f;
+    if (base + l < deg) {
+      j = colidx[k0 + base + l];
+      if (TRANSPOSE) sj = 1.f / (float)(rowptr[j + 1] - rowptr[j]);
+    }
+    const int left = min(16, most - base);
+    for (int q0 = 0; q0 < left; q0 += U) {
+      uint2 v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int jq = __shfl_sync(0xffffffffu, j, q0 + u, 16);
+        v[u] = make_uint2(0u, 0u);
+        if (base + q0 + u < deg) v[u] = *reinterpret_cast<const uint2 *>(in + (int64_t)jq * ldi + 4 * l);
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].x));
+        float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].y));
+        if (TRANSPOSE) {
+          const float sq = __shfl_sync(0xffffffffu, sj, q0 + u, 16);
+          lo.x *= sq; lo.y *= sq; hi.x *= sq; hi.y *= sq;
+        }
+        if (base + q0 + u < deg) {
+          acc.x += lo.x; acc.y += lo.y; acc.z += hi.x; acc.w += hi.y;
+        }
+      }
+    }
+  }
   if (node >= N) return;
-  const int k0 = rowptr[node], k1 = rowptr[node + 1];
-  float a0 = 0.f, a1 = 0.f;
-  for (int k = k0; k < k1; k++) {
-    const int j = colidx[k];
-    float v0, v1;
-    if (inf) {
-      const float2 v = *reinterpret_cast<const float2 *>(inf + (int64_t)j * HID + 2 * lane);
-      v0 = v.x; v1 = v.y;
-    } else {
-      const __nv_bfloat162 v = *reinterpret_cast<const __nv_bfloat162 *>(in + (int64_t)j * ldi + 2 * lane);
-      v0 = __bfloat162float(v.x); v1 = __bfloat162float(v.y);
-    }
-    if (transpose) {
-      const float s = 1.f / (float)(rowptr[j + 1] - rowptr[j]);
-      v0 *= s; v1 *= s;
-    }
-    a0 += v0; a1 += v1;
-  }
-  if (!transpose) {
-    const float s = 1.f / (float)(k1 - k0);
-    a0 *= s; a1 *= s;
-  }
-  if (outb) {
-    __nv_bfloat162 o;
-    o.x = __float2bfloat16(a0); o.y = __float2bfloat16(a1);
-    *reinterpret_cast<__nv_bfloat162 *>(outb + (int64_t)node * ldo + 2 * lane) = o;
-  }
-  if (outf) {
-    outf[(int64_t)node * HID + 2 * lane] += a0;
-    outf[(int64_t)node * HID + 2 * lane + 1] += a1;
+  if (TRANSPOSE) {
+    float4 *o = reinterpret_cast<float4 *>(outf + (int64_t)node * HID) + l;
+    float4 t = *o;
+    t.x += acc.x; t.y += acc.y; t.z += acc.z; t.w += acc.w;
+    *o = t;
+  } else {
+    const float sc = 1.f / (float)deg;
+    __nv_bfloat162 o[2];
+    o[0] = __floats2bfloat162_rn(acc.x * sc, acc.y * sc);
+    o[1] = __floats2bfloat162_rn(acc.z * sc, acc.w * sc);
+    *reinterpret_cast<uint2 *>(outb + (int64_t)node * ldo + 4 * l) = *reinterpret_cast<const uint2 *>(o);
   }
 }
 
@@ -337,11 +359,11 @@ __global__ void k_loss(int64_t count, const float *__restrict__ y, const float *
 
 __global__ void k_sum_partials(int n, const float *__restrict__ partial, float *__restrict__ out)
 {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float s = 0.f;
-    for (int i = 0; i < n; i++) s += partial[i];
-    out[0] = s;
-  }
+  float s = 0.f;   // one warp
+  for (int i = threadIdx.x; i < n; i += 32) s += partial[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) out[0] = s;
 }
 
 // dZ = dH * (Z > 0) (FP32 and BF16)
@@ -355,65 +377,135 @@ __global__ void k_relu_back(int64_t count, const float *__restrict__ dh, const f
   }
 }
 
+template <int T>
+__device__ __forceinline__ void load_row(float (&v)[T], const float *p)
+{
+  if constexpr (T == 2) {
+    const float2 t = *reinterpret_cast<const float2 *>(p);
+    v[0] = t.x; v[1] = t.y;
+  } else {
+    static_assert(T % 4 == 0, "16-byte pieces");
+#pragma unroll
+    for (int i = 0; i < T; i += 4) {
+      const float4 t = *reinterpret_cast<const float4 *>(p + i);
+      v[i] = t.x; v[i + 1] = t.y; v[i + 2] = t.z; v[i + 3] = t.w;
+    }
+  }
+}
+
 // weight gradient partials: part[chunk][k][o] = sum_{rows of chunk} A[r][k] dZ[r][o]
 // (A bf16 with row stride lda, dZ FP32 N x NO), plus the bias partial in the
-// extra row k = K.  Threads own (k, o) pairs; rows are walked in order.
-template <int K, int NO>
-__global__ void __launch_bounds__(256)
+// extra row k = K.  FP32 sums, rows in order.  A thread owns TK x TO outputs, so
+// a row costs it TK + TO shared-memory words for TK TO FMAs; a warp takes four
+// k-tiles by eight o-tiles, whose 16-byte reads are broadcasts without conflicts.
+// The next 32 rows are on their way from memory while these are added.  At 64 wide
+// layers bound by the FP32 FMA rate (66 us at 275,000 rows); a thread per output,
+// two shared-memory words for each FMA, took 475; now 113.
+constexpr int WG_ROWS = 32, WG_CHUNKS = 2 * 148;
+template <int K, int NO, int TK, int TO>
+__global__ void __launch_bounds__(256, 2)
 k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const float *__restrict__ dZ,
         float *__restrict__ part)
 {
-  constexpr int PAIRS = (K + 1) * NO;
-  __shared__ float sa[32][K + 1];
-  __shared__ float sz[32][NO];
+  static_assert((K / TK) * (NO / TO) == 256 && (NO / TO) % 8 == 0 && (K / TK) % 4 == 0, "tiles of 256 threads");
+  constexpr int WO = NO / TO / 8;                        // warps along o
+  constexpr int A8 = WG_ROWS * K / 8, Z4 = WG_ROWS * NO / 4;   // 16-byte pieces of a stage
+  constexpr int NA = (A8 + 255) / 256, NZ = (Z4 + 255) / 256;
+  __shared__ __align__(16) float sa[WG_ROWS][K];
+  __shared__ __align__(16) float sz[WG_ROWS][NO];
   const int r_begin = blockIdx.x * rows_per_chunk;
   const int r_end = min(Npad, r_begin + rows_per_chunk);
-  float acc[(PAIRS + 255) / 256];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kt = ((warp / WO) * 4 + (lane >> 3)) * TK, ot = ((warp % WO) * 8 + (lane & 7)) * TO;
+  float acc[TK][TO] = {}, bias[TO] = {};
+  uint4 pa[NA];
+  float4 pz[NZ];
+  // rows r0.. of the chunk into registers (zeros past its end)
+  auto fetch = [&](int r0) {
 #pragma unroll
-  for (int q = 0; q < (PAIRS + 255) / 256; q++) acc[q] = 0.f;
-  for (int r0 = r_begin; r0 < r_end; r0 += 32) {
-    const int nr = min(32, r_end - r0);
-    for (int i = threadIdx.x; i < 32 * K; i += 256) {
-      const int rr = i / K, kk = i % K;
-      sa[rr][kk] = (rr < nr) ? __bfloat162float(A[(int64_t)(r0 + rr) * lda + kk]) : 0.f;
+    for (int i = 0; i < NA; i++) {
+      const int q = i * 256 + threadIdx.x, rr = q / (K / 8), cc = q % (K / 8) * 8;
+      pa[i] = make_uint4(0u, 0u, 0u, 0u);
+      if (q < A8 && r0 + rr < r_end) pa[i] = *reinterpret_cast<const uint4 *>(A + (int64_t)(r0 + rr) * lda + cc);
     }
-    for (int i = threadIdx.x; i < 32; i += 256) sa[i][K] = (i < nr) ? 1.f : 0.f;
-    for (int i = threadIdx.x; i < 32 * NO; i += 256) {
-      const int rr = i / NO, oo = i % NO;
-      sz[rr][oo] = (rr < nr) ? dZ[(int64_t)(r0 + rr) * NO + oo] : 0.f;
+#pragma unroll
+    for (int i = 0; i < NZ; i++) {
+      const int q = i * 256 + threadIdx.x, rr = q / (NO / 4), cc = q % (NO / 4) * 4;
+      pz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (q < Z4 && r0 + rr < r_end) pz[i] = *reinterpret_cast<const float4 *>(dZ + (int64_t)(r0 + rr) * NO + cc);
+    }
+  };
+  fetch(r_begin);
+  for (int r0 = r_begin; r0 < r_end; r0 += WG_ROWS) {
+#pragma unroll
+    for (int i = 0; i < NA; i++) {
+      const int q = i * 256 + threadIdx.x, rr = q / (K / 8), cc = q % (K / 8) * 8;
+      if (q < A8) {
+        const uint32_t w[4] = {pa[i].x, pa[i].y, pa[i].z, pa[i].w};
+        float2 f[4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) f[e] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[e]));
+        *reinterpret_cast<float4 *>(&sa[rr][cc]) = make_float4(f[0].x, f[0].y, f[1].x, f[1].y);
+        *reinterpret_cast<float4 *>(&sa[rr][cc + 4]) = make_float4(f[2].x, f[2].y, f[3].x, f[3].y);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NZ; i++) {
+      const int q = i * 256 + threadIdx.x;
+      if (q < Z4) *reinterpret_cast<float4 *>(&sz[q / (NO / 4)][q % (NO / 4) * 4]) = pz[i];
     }
     __syncthreads();
+    if (r0 + WG_ROWS < r_end) fetch(r0 + WG_ROWS);
+#pragma unroll 4
+    for (int rr = 0; rr < WG_ROWS; rr++) {
+      float a[TK], z[TO];
+      load_row<TK>(a, &sa[rr][kt]);
+      load_row<TO>(z, &sz[rr][ot]);
 #pragma unroll
-    for (int q = 0; q < (PAIRS + 255) / 256; q++) {
-      const int pidx = q * 256 + threadIdx.x;
-      if (pidx < PAIRS) {
-        const int kk = pidx / NO, oo = pidx % NO;
-        float s = acc[q];
-        for (int rr = 0; rr < 32; rr++) s = fmaf(sa[rr][kk], sz[rr][oo], s);
-        acc[q] = s;
+      for (int i = 0; i < TK; i++)
+#pragma unroll
+        for (int o = 0; o < TO; o++) acc[i][o] = fmaf(a[i], z[o], acc[i][o]);
+      if (warp < WO) {
+#pragma unroll
+        for (int o = 0; o < TO; o++) bias[o] += z[o];
       }
     }
     __syncthreads();
   }
+  float *p = part + (int64_t)blockIdx.x * (K + 1) * NO;
 #pragma unroll
-  for (int q = 0; q < (PAIRS + 255) / 256; q++) {
-    const int pidx = q * 256 + threadIdx.x;
-    if (pidx < PAIRS) part[(int64_t)blockIdx.x * PAIRS + pidx] = acc[q];
+  for (int i = 0; i < TK; i++)
+#pragma unroll
+    for (int o = 0; o < TO; o++) p[(kt + i) * NO + ot + o] = acc[i][o];
+  if (kt == 0) {
+#pragma unroll
+    for (int o = 0; o < TO; o++) p[K * NO + ot + o] = bias[o];
   }
 }
 
-// sum the chunk partials in order into the gradient blocks (W then bias)
-__global__ void k_wgrad_reduce(int nchunks, int K, int NO, const float *__restrict__ part, float *__restrict__ gW,
-                               float *__restrict__ gb)
+// sum the chunk partials into the gradient blocks (W then bias): a CTA takes 32
+// outputs, warp w the chunks congruent to w modulo 8, then the eight sums in
+// order.  One thread per output over all chunks took 99 us a layer at 464 chunks; now 5.
+__global__ void __launch_bounds__(256)
+k_wgrad_reduce(int nchunks, int K, int NO, const float *__restrict__ part, float *__restrict__ gW,
+               float *__restrict__ gb)
 {
-  const int pidx = blockIdx.x * blockDim.x + threadIdx.x;
+  __shared__ float sh[8][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int PAIRS = (K + 1) * NO;
-  if (pidx >= PAIRS) return;
+  const int pidx = blockIdx.x * 32 + lane;
   float s = 0.f;
-  for (int c = 0; c < nchunks; c++) s += part[(int64_t)c * PAIRS + pidx];
-  const int kk = pidx / NO, oo = pidx % NO;
-  if (kk < K) gW[kk * NO + oo] = s;
-  else gb[oo] = s;
+  if (pidx < PAIRS) {
+#pragma unroll 8
+    for (int c = warp; c < nchunks; c += 8) s += part[(int64_t)c * PAIRS + pidx];
+  }
+  sh[warp][lane] = s;
+  __syncthreads();
+  if (warp != 0 || pidx >= PAIRS) return;
+#pragma unroll
+  for (int w = 1; w < 8; w++) s += sh[w][lane];
+  if (pidx < K * NO) gW[pidx] = s;
+  else gb[pidx - K * NO] = s;
 }
 
 // dH_prev = dH (residual) + dCat[:, :HID]; dM (mean part) -> scaled BF16 for the transposed aggregation
@@ -477,6 +569,9 @@ inline void weight_shape(int w, int &K, int &NO)
 inline int weight_off(const PLayout &L, int w) { return w == 0 ? L.We : (w <= LAYERS ? L.W[w - 1] : L.Wd); }
 inline int bias_off(const PLayout &L, int w) { return w == 0 ? L.be : (w <= LAYERS ? L.b[w - 1] : L.bd); }
 
+// rows of one CTA of the weight gradient: whole stages, two CTAs per SM at most
+inline int wgrad_rows(int Npad) { return (Npad + WG_CHUNKS * WG_ROWS - 1) / (WG_CHUNKS * WG_ROWS) * WG_ROWS; }
+
 int refresh_bf16(cfdgpu_mpnn *m)
 {
   for (int w = 0; w < LAYERS + 2; w++) {
@@ -499,9 +594,9 @@ int forward(cfdgpu_mpnn *m, const bf16 *X)
   gemm_bf16<FIN, HID><<<gridg, 128, 0, s>>>(Np, X, m->Wb + m->wb_off[1], m->P + L.be, m->Ze);
   k_act<<<grid1(cnt), 256, 0, s>>>(cnt, m->Ze, nullptr, m->Hf[0], m->Cat[0], 2 * HID);
   for (int l = 0; l < LAYERS; l++) {
-    const int aggGrid = (int)((m->N * 32LL + 255) / 256);
-    k_mean_agg<<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->Cat[l], 2 * HID, m->Cat[l] + HID, 2 * HID,
-                                       nullptr, nullptr, 0);
+    const int aggGrid = (int)((m->N * 16LL + 255) / 256);
+    k_mean_agg<false><<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->Cat[l], 2 * HID, m->Cat[l] + HID,
+                                              2 * HID, nullptr);
     gemm_bf16<2 * HID, HID><<<gridg, 128, 0, s>>>(Np, m->Cat[l], m->Wb + m->wb_off[2 * (l + 1) + 1], m->P + L.b[l], m->Z[l]);
     bf16 *next = (l + 1 < LAYERS) ? m->Cat[l + 1] : m->H3b;
     const int ldn = (l + 1 < LAYERS) ? 2 * HID : HID;
@@ -516,12 +611,12 @@ int wgrad(cfdgpu_mpnn *m, int w, const bf16 *A, int lda, const float *dZ)
   cudaStream_t s = m->g.stream;
   int K, NO;
   weight_shape(w, K, NO);
-  const int rpc = m->Npad / m->nchunks;
-  if (w == 0) k_wgrad<FIN, HID><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
-  else if (w <= LAYERS) k_wgrad<2 * HID, HID><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
-  else k_wgrad<HID, FOUT><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
+  const int rpc = wgrad_rows(m->Npad);
+  if (w == 0) k_wgrad<FIN, HID, 2, 2><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
+  else if (w <= LAYERS) k_wgrad<2 * HID, HID, 8, 4><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
+  else k_wgrad<HID, FOUT, 2, 2><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
   const int pairs = (K + 1) * NO;
-  k_wgrad_reduce<<<(pairs + 255) / 256, 256, 0, s>>>(m->nchunks, K, NO, m->partial, m->G + weight_off(m->L, w),
+  k_wgrad_reduce<<<(pairs + 31) / 32, 256, 0, s>>>(m->nchunks, K, NO, m->partial, m->G + weight_off(m->L, w),
                                                      m->G + bias_off(m->L, w));
   return cudaGetLastError() == cudaSuccess ? 0 : CFDGPU_ECUDA;
 }
@@ -548,8 +643,8 @@ int backward(cfdgpu_mpnn *m, const bf16 *X, const float *T, float *loss_dev)
     // dCat = dZ W_l^T  (W_l stored K x NO = 128 x 64)
     gemm_bf16<HID, 2 * HID><<<gridg, 128, 0, s>>>(Np, m->dZb, m->Wb + m->wb_off[2 * (l + 1)], nullptr, m->dCat);
     k_split_dcat<<<grid1(cnt), 256, 0, s>>>(cnt, m->dCat, m->dH, m->dMs);
-    const int aggGrid = (int)((m->N * 32LL + 255) / 256);
-    k_mean_agg<<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->dMs, HID, nullptr, 0, nullptr, m->dH, 1);
+    const int aggGrid = (int)((m->N * 16LL + 255) / 256);
+    k_mean_agg<true><<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->dMs, HID, nullptr, 0, m->dH);
   }
   k_relu_back<<<grid1(cnt), 256, 0, s>>>(cnt, m->dH, m->Ze, m->dZ, m->dZb);
   if ((rc = wgrad(m, 0, X, FIN, m->dZ))) return rc;
@@ -677,8 +772,7 @@ int cfdgpu_mpnn_create(cfdgpu_handle *h, uint64_t seed, cfdgpu_mpnn **out)
       (rc = dalloc(m, &m->dCat, (size_t)Np * 2 * HID)) || (rc = dalloc(m, &m->mask, (size_t)Np * FOUT)) ||
       (rc = dalloc(m, &m->lossbuf, 256)))
     return rc;
-  m->nchunks = std::max(1, std::min(512, Np / 256));
-  while (Np % m->nchunks) m->nchunks--;
+  m->nchunks = (Np + wgrad_rows(Np) - 1) / wgrad_rows(Np);
   if ((rc = dalloc(m, &m->partial, (size_t)m->nchunks * (2 * HID + 1) * HID))) return rc;
   k_mask<<<(m->N + 255) / 256, 256, 0, m->g.stream>>>(m->N, m->g.ndof, m->g.fixmask, m->mask);
   m->graphs.push_back({m->g, m->N, m->mask, m->xlo, m->xinv});
