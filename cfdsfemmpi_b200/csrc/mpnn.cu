@@ -65,18 +65,15 @@ struct cfdgpu_mpnn {
   int64_t step = 0;
   // activations
   bf16 *X = nullptr;                 // N x FIN
-  float *Ze = nullptr;               // N x HID (encoder pre-activation)
-  float *Hf[LAYERS + 1];             // N x HID FP32
+  float *H = nullptr;                // N x HID FP32, h_l while layer l runs
+  uint64_t *pos[LAYERS + 1];         // N words: bit c of row i is set where the pre-activation is positive
   bf16 *Cat[LAYERS];                 // N x 2HID: [h_{l-1}, mean]
-  float *Z[LAYERS];                  // N x HID pre-activation
   bf16 *H3b = nullptr;               // N x HID (decoder input)
   float *Y = nullptr;                // N x FOUT
   // backward scratch
-  float *dH = nullptr, *dZ = nullptr, *dY = nullptr;
-  bf16 *dZb = nullptr, *dYb = nullptr, *dMs = nullptr;
-  float *dCat = nullptr;             // N x 2HID
+  float *dH = nullptr, *dY = nullptr;
+  bf16 *dYb = nullptr, *dMs = nullptr;
   float *partial = nullptr;          // per-CTA weight-gradient partials
-  int nchunks = 0;
   float *lossbuf = nullptr;
   // normalisation
   float in_scale[8] = {1, 1, 1, 1, 1, 1, 1, 1}, out_scale[4] = {1, 1, 1, 1};
@@ -85,14 +82,15 @@ struct cfdgpu_mpnn {
   std::vector<bf16 *> sx;
   std::vector<float *> st;
   float *mask = nullptr;             // N x FOUT, 1 on free dofs
+  float *deginv = nullptr;           // N, 1 / neighbours
   // the mesh graphs samples live on: [0] the graph of the handle the network
   // was created on (the one its predictions serve), then graphs of other
   // handles whose samples train the same weights (at most as many nodes);
-  // g, N, mask, xlo, xinv above hold the graph in use
+  // g, N, mask, deginv, xlo, xinv above hold the graph in use
   struct Graph {
     cfdgpu::GraphView g;
     int N;
-    float *mask;
+    float *mask, *deginv;
     double3 xlo, xinv;
   };
   std::vector<Graph> graphs;
@@ -124,9 +122,20 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// C[Npad x NO] = A[Npad x K] (bf16, row-major) * W (bf16, given as Wt = NO x K
-// row-major, i.e. the "col" operand of mma.sync) + bias (optional), FP32
-// accumulation and FP32 output.  One warp computes 16 rows x NO columns
+// Dense layers: acc[Npad x NO] = A[Npad x K] * W, bf16 operands (W given as
+// Wt = NO x K row-major, i.e. the "col" operand of mma.sync), FP32 accumulation,
+// and what follows done on the accumulators.  FORM:
+//   PLAIN  C = acc + bias (optional); A bf16
+//   LAYER  z = acc + bias; h += relu(z) (h = relu(z) with first), its bf16 copy
+//          into bout (leading dimension ldb), the signs of z into pos; A bf16
+//   BACK   A = dH where pos, rounded to bf16; then dH += acc[:, :HID] in place and
+//          dM = bf16(acc[:, HID:]); a warp's rows of dH are its own
+// Bound by memory.  With the activation, its derivative and the split of the
+// gradient as passes of their own (z, dz and the gradient of the concatenation
+// written and read back) a layer took 75 + 41 us forward and 41 + 108 backward at
+// 274,625 nodes; now 61 and 52.
+//
+// One warp computes 16 rows x NO columns
 // (NO/8 m16n8k16 tiles per k-step of 16); 4 warps per CTA, each CTA walking
 // 64-row tiles with a grid stride.  The weights are staged in shared memory
 // once per CTA with rows padded to K + 8 elements, so the eight row groups of
@@ -136,19 +145,32 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
 // memory with 16-byte asynchronous copies (padded the same way) and reads its
 // fragments from there: fragment loads straight from global memory touch
 // eight rows per instruction and bound the kernel at L1.
-template <int K, int NO>
+enum GemmForm { PLAIN, LAYER, BACK };
+struct GemmIO {
+  const bf16 *A;        // PLAIN, LAYER
+  const bf16 *Wt;
+  const float *bias;    // PLAIN (or null), LAYER
+  float *C;             // PLAIN
+  float *h;             // LAYER: h; BACK: dH
+  bf16 *b;              // LAYER: bout; BACK: dM
+  int ldb;              // LAYER
+  bool first;           // LAYER
+  uint64_t *pos;        // LAYER: out; BACK: in
+};
+template <int K, int NO, int FORM>
 __global__ void __launch_bounds__(128)
-gemm_bf16(int Npad, const bf16 *__restrict__ A, const bf16 *__restrict__ Wt, const float *__restrict__ bias,
-          float *__restrict__ C)
+gemm_bf16(int Npad, const GemmIO g)
 {
   constexpr int KP = K + 8;
   constexpr int CPR = K / 8;                    // 16-byte chunks per row of A
   static_assert(K % 8 == 0, "rows of A in 16-byte chunks");
+  static_assert(FORM != LAYER || NO == HID, "");
+  static_assert(FORM != BACK || (K == HID && NO == 2 * HID), "");
   __shared__ __align__(16) bf16 sW[NO * KP];
   __shared__ __align__(16) bf16 sA[4][16 * KP];
   for (int i = threadIdx.x; i < NO * K / 2; i += blockDim.x) {
     const int rr = (2 * i) / K, cc = (2 * i) % K;
-    *reinterpret_cast<uint32_t *>(sW + rr * KP + cc) = reinterpret_cast<const uint32_t *>(Wt)[i];
+    *reinterpret_cast<uint32_t *>(sW + rr * KP + cc) = reinterpret_cast<const uint32_t *>(g.Wt)[i];
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -157,14 +179,36 @@ gemm_bf16(int Npad, const bf16 *__restrict__ A, const bf16 *__restrict__ Wt, con
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
   const int r0 = tile * ROWS_PER_CTA + warp * 16;
   bf16 *const wa = sA[warp];
-  for (int q = lane; q < 16 * CPR; q += 32) {
-    const int rr = q / CPR, cc = (q % CPR) * 8;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(wa + rr * KP + cc)),
-                 "l"(A + (int64_t)(r0 + rr) * K + cc)
-                 : "memory");
+  if constexpr (FORM == BACK) {
+#pragma unroll
+    for (int i = 0; i < 16 * K / 4 / 32; i++) {
+      const int q = i * 32 + lane, rr = q / (K / 4), cc = q % (K / 4) * 4;
+      const float4 v = *reinterpret_cast<const float4 *>(g.h + (int64_t)(r0 + rr) * K + cc);
+      const uint32_t on = (uint32_t)(g.pos[r0 + rr] >> cc);
+      __nv_bfloat162 o[2];
+      o[0] = __floats2bfloat162_rn(on & 1u ? v.x : 0.f, on & 2u ? v.y : 0.f);
+      o[1] = __floats2bfloat162_rn(on & 4u ? v.z : 0.f, on & 8u ? v.w : 0.f);
+      *reinterpret_cast<uint2 *>(wa + rr * KP + cc) = *reinterpret_cast<const uint2 *>(o);
+    }
+  } else {
+    for (int q = lane; q < 16 * CPR; q += 32) {
+      const int rr = q / CPR, cc = (q % CPR) * 8;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(wa + rr * KP + cc)),
+                   "l"(g.A + (int64_t)(r0 + rr) * K + cc)
+                   : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncwarp();
+  // the FP32 rows that the results are added to, on their way during the product
+  float2 h0[2][HID / 8] = {};
+  if (FORM == BACK || (FORM == LAYER && !g.first)) {
+#pragma unroll
+    for (int half = 0; half < 2; half++)
+#pragma unroll
+      for (int t = 0; t < HID / 8; t++)
+        h0[half][t] = *reinterpret_cast<const float2 *>(g.h + (int64_t)(r0 + gq + 8 * half) * HID + t * 8 + 2 * tq);
+  }
   float acc[NO / 8][4];
 #pragma unroll
   for (int t = 0; t < NO / 8; t++) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
@@ -186,13 +230,36 @@ gemm_bf16(int Npad, const bf16 *__restrict__ A, const bf16 *__restrict__ Wt, con
     }
   }
 #pragma unroll
-  for (int t = 0; t < NO / 8; t++) {
-    const int c = t * 8 + 2 * tq;
-    const float b0 = bias ? bias[c] : 0.f, b1 = bias ? bias[c + 1] : 0.f;
-    float2 v0 = make_float2(acc[t][0] + b0, acc[t][1] + b1);
-    float2 v1 = make_float2(acc[t][2] + b0, acc[t][3] + b1);
-    *reinterpret_cast<float2 *>(C + (int64_t)(r0 + gq) * NO + c) = v0;
-    *reinterpret_cast<float2 *>(C + (int64_t)(r0 + gq + 8) * NO + c) = v1;
+  for (int half = 0; half < 2; half++) {
+    const int64_t r = r0 + gq + 8 * half;
+    uint64_t on = 0;
+#pragma unroll
+    for (int t = 0; t < NO / 8; t++) {
+      const int c = t * 8 + 2 * tq;
+      float2 v = make_float2(acc[t][2 * half], acc[t][2 * half + 1]);
+      if constexpr (FORM != BACK) {
+        v.x += g.bias ? g.bias[c] : 0.f;
+        v.y += g.bias ? g.bias[c + 1] : 0.f;
+      }
+      if constexpr (FORM == PLAIN) {
+        *reinterpret_cast<float2 *>(g.C + r * NO + c) = v;
+      } else if constexpr (FORM == LAYER) {
+        on |= (uint64_t)((v.x > 0.f ? 1u : 0u) | (v.y > 0.f ? 2u : 0u)) << c;
+        v.x = fmaxf(v.x, 0.f) + h0[half][t].x;
+        v.y = fmaxf(v.y, 0.f) + h0[half][t].y;
+        *reinterpret_cast<float2 *>(g.h + r * HID + c) = v;
+        *reinterpret_cast<__nv_bfloat162 *>(g.b + r * g.ldb + c) = __floats2bfloat162_rn(v.x, v.y);
+      } else if (c < HID) {
+        *reinterpret_cast<float2 *>(g.h + r * HID + c) = make_float2(h0[half][t].x + v.x, h0[half][t].y + v.y);
+      } else {
+        *reinterpret_cast<__nv_bfloat162 *>(g.b + r * HID + c - HID) = __floats2bfloat162_rn(v.x, v.y);
+      }
+    }
+    if constexpr (FORM == LAYER) {
+      on |= __shfl_xor_sync(0xffffffffu, on, 1);
+      on |= __shfl_xor_sync(0xffffffffu, on, 2);
+      if (tq == 0) g.pos[r] = on;
+    }
   }
   // every lane has read its fragments before the next tile's copy lands
   __syncwarp();
@@ -202,84 +269,84 @@ gemm_bf16(int Npad, const bf16 *__restrict__ A, const bf16 *__restrict__ Wt, con
 // CTAs of gemm_bf16 for Npad rows: one per 64-row tile, at most 8 per SM
 inline int gemm_grid(int Npad) { return std::max(1, std::min(Npad / ROWS_PER_CTA, 148 * 8)); }
 
-// h = relu(z) (encoder) or h = hprev + relu(z) (residual layers); writes the
-// FP32 result and its BF16 copy into column block [0, HID) of the next
-// layer's concatenated input (ld = 2*HID) or into a plain N x HID buffer.
-__global__ void k_act(int64_t count, const float *__restrict__ z, const float *__restrict__ hprev,
-                      float *__restrict__ hout, bf16 *__restrict__ bout, int ldb)
-{
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-    const float v = fmaxf(z[i], 0.f) + (hprev ? hprev[i] : 0.f);
-    hout[i] = v;
-    if (bout) bout[(i / HID) * ldb + (i % HID)] = __float2bfloat16(v);
-  }
-}
-
 // mean over the node's neighbourhood: out[i][c] = (1/deg_i) sum_j in[j][c],
-// neighbours in column order.  Half a warp per node, four channels per lane;
-// the 16 lanes load 16 column indices at once and hand them round, and the rows
-// of eight neighbours are in flight together.  T = bf16 input with leading
-// dimension ldi; the mean goes to outb as bf16 (leading dimension ldo).  TRANSPOSE
-// divides the inputs by their own node's degree instead (the transpose of the
-// mean on the symmetric pattern) and adds the sum to outf (FP32).
-// Bound by the rows' way from L2 and L1 (27 x 128 bytes a node on a hexahedral
-// mesh).  One load at a time after its own index took 202 us at
-// 274,625 nodes and 27 neighbours; now 144 (191 transposed).
+// neighbours in column order.  Eight lanes per node, eight channels (16 bytes) per
+// lane; the lanes load eight column indices at once and hand them round, and the
+// rows of eight neighbours are in flight together.  in has leading dimension ldi;
+// the mean goes to outb as bf16 (leading dimension ldo).  TRANSPOSE multiplies the
+// inputs by their own node's 1/deg instead (the transpose of the mean on the
+// symmetric pattern) and adds the sum to outf (FP32).
+// Bound by instruction issue (83 % of its peak with four channels a lane, L1 39 %, L2
+// 11 %: 144 us at 274,625 nodes and 27 neighbours, 191 transposed, where each
+// neighbour's degree was looked up and divided by; one load at a time after its own
+// index took 202); now 84 and 100.
 template <bool TRANSPOSE>
-__global__ void __launch_bounds__(256, 5)
-k_mean_agg(int N, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx, const bf16 *__restrict__ in,
-           int ldi, bf16 *__restrict__ outb, int ldo, float *__restrict__ outf)
+__global__ void __launch_bounds__(256, 4)
+k_mean_agg(int N, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
+           const float *__restrict__ deginv, const bf16 *__restrict__ in, int ldi, bf16 *__restrict__ outb, int ldo,
+           float *__restrict__ outf)
 {
   constexpr int U = 8;
-  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-  const int l = threadIdx.x & 15;
+  const int node = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+  const int l = threadIdx.x & 7;
   const int k0 = (node < N) ? rowptr[node] : 0, deg = (node < N) ? rowptr[node + 1] - k0 : 0;
-  const int other = __shfl_xor_sync(0xffffffffu, deg, 16);
-  const int most = max(deg, other);   // both halves of the warp take the same steps
-  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int base = 0; base < most; base += 16) {
-    int j = 0;
+  // the four nodes of a warp take the same steps
+  int most = max(deg, __shfl_xor_sync(0xffffffffu, deg, 8)), least = min(deg, __shfl_xor_sync(0xffffffffu, deg, 8));
+  most = max(most, __shfl_xor_sync(0xffffffffu, most, 16));
+  least = min(least, __shfl_xor_sync(0xffffffffu, least, 16));
+  const bf16 *const col = in + 8 * l;
+  float acc[8] = {};
+  for (int base = 0; base < most; base += U) {
+    int j = 0;             // a place past the end reads row 0 and is not added
+    if (base + l < deg) j = colidx[k0 + base + l];
     float sj = 1.f;
-    if (base + l < deg) {
-      j = colidx[k0 + base + l];
-      if (TRANSPOSE) sj = 1.f / (float)(rowptr[j + 1] - rowptr[j]);
-    }
-    const int left = min(16, most - base);
-    for (int q0 = 0; q0 < left; q0 += U) {
-      uint2 v[U];
+    if (TRANSPOSE) sj = deginv[j];
+    uint4 v[U];
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int jq = __shfl_sync(0xffffffffu, j, q0 + u, 16);
-        v[u] = make_uint2(0u, 0u);
-        if (base + q0 + u < deg) v[u] = *reinterpret_cast<const uint2 *>(in + (int64_t)jq * ldi + 4 * l);
+    for (int u = 0; u < U; u++)
+      v[u] = *reinterpret_cast<const uint4 *>(col + (int64_t)__shfl_sync(0xffffffffu, j, u, 8) * ldi);
+    const bool whole = base + U <= least;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+      float f[8];
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        f[2 * e] = __uint_as_float(w[e] << 16);
+        f[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u);
       }
+      if (TRANSPOSE) {
+        const float sq = __shfl_sync(0xffffffffu, sj, u, 8);
 #pragma unroll
-      for (int u = 0; u < U; u++) {
-        float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].x));
-        float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&v[u].y));
-        if (TRANSPOSE) {
-          const float sq = __shfl_sync(0xffffffffu, sj, q0 + u, 16);
-          lo.x *= sq; lo.y *= sq; hi.x *= sq; hi.y *= sq;
-        }
-        if (base + q0 + u < deg) {
-          acc.x += lo.x; acc.y += lo.y; acc.z += hi.x; acc.w += hi.y;
-        }
+        for (int e = 0; e < 8; e++) f[e] *= sq;
+      }
+      if (whole || base + u < deg) {
+#pragma unroll
+        for (int e = 0; e < 8; e++) acc[e] += f[e];
       }
     }
   }
   if (node >= N) return;
   if (TRANSPOSE) {
-    float4 *o = reinterpret_cast<float4 *>(outf + (int64_t)node * HID) + l;
-    float4 t = *o;
-    t.x += acc.x; t.y += acc.y; t.z += acc.z; t.w += acc.w;
-    *o = t;
+    float4 *o = reinterpret_cast<float4 *>(outf + (int64_t)node * HID + 8 * l);
+    float4 t0 = o[0], t1 = o[1];
+    t0.x += acc[0]; t0.y += acc[1]; t0.z += acc[2]; t0.w += acc[3];
+    t1.x += acc[4]; t1.y += acc[5]; t1.z += acc[6]; t1.w += acc[7];
+    o[0] = t0;
+    o[1] = t1;
   } else {
-    const float sc = 1.f / (float)deg;
-    __nv_bfloat162 o[2];
-    o[0] = __floats2bfloat162_rn(acc.x * sc, acc.y * sc);
-    o[1] = __floats2bfloat162_rn(acc.z * sc, acc.w * sc);
-    *reinterpret_cast<uint2 *>(outb + (int64_t)node * ldo + 4 * l) = *reinterpret_cast<const uint2 *>(o);
+    const float sc = deginv[node];
+    __nv_bfloat162 o[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) o[e] = __floats2bfloat162_rn(acc[2 * e] * sc, acc[2 * e + 1] * sc);
+    *reinterpret_cast<uint4 *>(outb + (int64_t)node * ldo + 8 * l) = *reinterpret_cast<const uint4 *>(o);
   }
+}
+
+__global__ void k_deg_inv(int N, const int32_t *__restrict__ rowptr, float *__restrict__ deginv)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < N) deginv[i] = 1.f / (float)(rowptr[i + 1] - rowptr[i]);
 }
 
 // input features of one sample / prediction
@@ -334,27 +401,39 @@ __global__ void k_mask(int N, int ndof, const uint8_t *__restrict__ fixmask, flo
 }
 
 // loss = sum mask (y - t)^2 / sum mask ; dY = 2 mask (y - t) / sum mask (BF16 copy
-// for the backward GEMM).  Deterministic: per-CTA partials, then one CTA.
-__global__ void k_loss(int64_t count, const float *__restrict__ y, const float *__restrict__ t,
-                       const float *__restrict__ mask, float inv_cnt, float *__restrict__ dy, bf16 *__restrict__ dyb,
-                       float *__restrict__ partial)
+// for the backward GEMM).  count is a multiple of 4.  Deterministic: per-CTA
+// partials, then one warp.  Bound by memory; 148 CTAs of 256 threads with one entry
+// at a time took 55 us at 274,688 x 16 entries, now 13.
+constexpr int LOSS_THREADS = 1024;
+__global__ void __launch_bounds__(LOSS_THREADS)
+k_loss(int64_t count, const float *__restrict__ y, const float *__restrict__ t, const float *__restrict__ mask,
+       float inv_cnt, float *__restrict__ dy, bf16 *__restrict__ dyb, float *__restrict__ partial)
 {
-  __shared__ float sh[256];
+  __shared__ float sh[LOSS_THREADS / 32];
   float s = 0.f;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-    const float d = (y[i] - t[i]) * mask[i];
-    s += d * d;
-    const float g = 2.f * d * inv_cnt;
-    dy[i] = g;
-    dyb[i] = __float2bfloat16(g);
+  for (int64_t i = (int64_t)blockIdx.x * LOSS_THREADS + threadIdx.x; i < count / 4; i += (int64_t)gridDim.x * LOSS_THREADS) {
+    const float4 a = reinterpret_cast<const float4 *>(y)[i], b = reinterpret_cast<const float4 *>(t)[i];
+    const float4 k = reinterpret_cast<const float4 *>(mask)[i];
+    const float d[4] = {(a.x - b.x) * k.x, (a.y - b.y) * k.y, (a.z - b.z) * k.z, (a.w - b.w) * k.w};
+    float g[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      s += d[e] * d[e];
+      g[e] = 2.f * d[e] * inv_cnt;
+    }
+    reinterpret_cast<float4 *>(dy)[i] = make_float4(g[0], g[1], g[2], g[3]);
+    __nv_bfloat162 o[2] = {__floats2bfloat162_rn(g[0], g[1]), __floats2bfloat162_rn(g[2], g[3])};
+    reinterpret_cast<uint2 *>(dyb)[i] = *reinterpret_cast<const uint2 *>(o);
   }
-  sh[threadIdx.x] = s;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = s;
   __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) partial[blockIdx.x] = sh[0] * inv_cnt;
+  if (threadIdx.x >= 32) return;
+  s = sh[threadIdx.x];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s * inv_cnt;
 }
 
 __global__ void k_sum_partials(int n, const float *__restrict__ partial, float *__restrict__ out)
@@ -364,17 +443,6 @@ __global__ void k_sum_partials(int n, const float *__restrict__ partial, float *
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if (threadIdx.x == 0) out[0] = s;
-}
-
-// dZ = dH * (Z > 0) (FP32 and BF16)
-__global__ void k_relu_back(int64_t count, const float *__restrict__ dh, const float *__restrict__ z,
-                            float *__restrict__ dz, bf16 *__restrict__ dzb)
-{
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-    const float v = (z[i] > 0.f) ? dh[i] : 0.f;
-    dz[i] = v;
-    dzb[i] = __float2bfloat16(v);
-  }
 }
 
 template <int T>
@@ -394,18 +462,21 @@ __device__ __forceinline__ void load_row(float (&v)[T], const float *p)
 }
 
 // weight gradient partials: part[chunk][k][o] = sum_{rows of chunk} A[r][k] dZ[r][o]
-// (A bf16 with row stride lda, dZ FP32 N x NO), plus the bias partial in the
-// extra row k = K.  FP32 sums, rows in order.  A thread owns TK x TO outputs, so
+// (A bf16 with row stride lda, dZ FP32 N x NO, taken where pos if that is given),
+// plus the bias partial in the extra row k = K.  FP32 sums, rows in order.  A thread owns TK x TO outputs, so
 // a row costs it TK + TO shared-memory words for TK TO FMAs; a warp takes four
 // k-tiles by eight o-tiles, whose 16-byte reads are broadcasts without conflicts.
 // The next 32 rows are on their way from memory while these are added.  At 64 wide
 // layers bound by the FP32 FMA rate (66 us at 275,000 rows); a thread per output,
-// two shared-memory words for each FMA, took 475; now 113.
-constexpr int WG_ROWS = 32, WG_CHUNKS = 2 * 148;
+// two shared-memory words for each FMA, took 475; now 113,
+// and 134 with the signs applied on the way (a pass of its own for that took 47).
+// CTAs per SM: the small layers are short of loads in flight, not of FMAs
+constexpr int WG_ROWS = 32;
+template <int OUTPUTS> constexpr int WG_CTAS = OUTPUTS == 32 ? 2 : 4;
 template <int K, int NO, int TK, int TO>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, WG_CTAS<TK * TO>)
 k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const float *__restrict__ dZ,
-        float *__restrict__ part)
+        const uint64_t *__restrict__ pos, float *__restrict__ part)
 {
   static_assert((K / TK) * (NO / TO) == 256 && (NO / TO) % 8 == 0 && (K / TK) % 4 == 0, "tiles of 256 threads");
   constexpr int WO = NO / TO / 8;                        // warps along o
@@ -420,6 +491,7 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
   float acc[TK][TO] = {}, bias[TO] = {};
   uint4 pa[NA];
   float4 pz[NZ];
+  uint32_t on[NZ];
   // rows r0.. of the chunk into registers (zeros past its end)
   auto fetch = [&](int r0) {
 #pragma unroll
@@ -432,7 +504,11 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
     for (int i = 0; i < NZ; i++) {
       const int q = i * 256 + threadIdx.x, rr = q / (NO / 4), cc = q % (NO / 4) * 4;
       pz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (q < Z4 && r0 + rr < r_end) pz[i] = *reinterpret_cast<const float4 *>(dZ + (int64_t)(r0 + rr) * NO + cc);
+      on[i] = 15u;
+      if (q < Z4 && r0 + rr < r_end) {
+        pz[i] = *reinterpret_cast<const float4 *>(dZ + (int64_t)(r0 + rr) * NO + cc);
+        if (pos) on[i] = (uint32_t)(pos[r0 + rr] >> cc);
+      }
     }
   };
   fetch(r_begin);
@@ -452,7 +528,10 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
 #pragma unroll
     for (int i = 0; i < NZ; i++) {
       const int q = i * 256 + threadIdx.x;
-      if (q < Z4) *reinterpret_cast<float4 *>(&sz[q / (NO / 4)][q % (NO / 4) * 4]) = pz[i];
+      const uint32_t o = on[i];
+      if (q < Z4)
+        *reinterpret_cast<float4 *>(&sz[q / (NO / 4)][q % (NO / 4) * 4]) =
+            make_float4(o & 1u ? pz[i].x : 0.f, o & 2u ? pz[i].y : 0.f, o & 4u ? pz[i].z : 0.f, o & 8u ? pz[i].w : 0.f);
     }
     __syncthreads();
     if (r0 + WG_ROWS < r_end) fetch(r0 + WG_ROWS);
@@ -508,17 +587,6 @@ k_wgrad_reduce(int nchunks, int K, int NO, const float *__restrict__ part, float
   else gb[pidx - K * NO] = s;
 }
 
-// dH_prev = dH (residual) + dCat[:, :HID]; dM (mean part) -> scaled BF16 for the transposed aggregation
-__global__ void k_split_dcat(int64_t count, const float *__restrict__ dcat, float *__restrict__ dh,
-                             bf16 *__restrict__ dm)
-{
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t r = i / HID, c = i % HID;
-    dh[i] += dcat[r * 2 * HID + c];
-    dm[i] = __float2bfloat16(dcat[r * 2 * HID + HID + c]);
-  }
-}
-
 __global__ void k_adam(int n, float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
                        float *__restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2)
 {
@@ -557,8 +625,6 @@ __global__ void k_write_delta(int N, int ndof, const float *__restrict__ y, floa
   }
 }
 
-inline int grid1(int64_t n, int bs = 256) { return (int)std::min<int64_t>((n + bs - 1) / bs, 148 * 32); }
-
 // weight index helpers: block order We, W[0..2], Wd
 inline void weight_shape(int w, int &K, int &NO)
 {
@@ -569,8 +635,12 @@ inline void weight_shape(int w, int &K, int &NO)
 inline int weight_off(const PLayout &L, int w) { return w == 0 ? L.We : (w <= LAYERS ? L.W[w - 1] : L.Wd); }
 inline int bias_off(const PLayout &L, int w) { return w == 0 ? L.be : (w <= LAYERS ? L.b[w - 1] : L.bd); }
 
-// rows of one CTA of the weight gradient: whole stages, two CTAs per SM at most
-inline int wgrad_rows(int Npad) { return (Npad + WG_CHUNKS * WG_ROWS - 1) / (WG_CHUNKS * WG_ROWS) * WG_ROWS; }
+// rows of one CTA of the weight gradient: whole stages, `ctas` CTAs per SM at most
+inline int wgrad_rows(int Npad, int ctas)
+{
+  const int most = ctas * 148 * WG_ROWS;
+  return (Npad + most - 1) / most * WG_ROWS;
+}
 
 int refresh_bf16(cfdgpu_mpnn *m)
 {
@@ -590,33 +660,34 @@ int forward(cfdgpu_mpnn *m, const bf16 *X)
   const int Np = m->Npad;
   const int gridg = gemm_grid(Np);
   const PLayout &L = m->L;
-  const int64_t cnt = (int64_t)Np * HID;
-  gemm_bf16<FIN, HID><<<gridg, 128, 0, s>>>(Np, X, m->Wb + m->wb_off[1], m->P + L.be, m->Ze);
-  k_act<<<grid1(cnt), 256, 0, s>>>(cnt, m->Ze, nullptr, m->Hf[0], m->Cat[0], 2 * HID);
+  gemm_bf16<FIN, HID, LAYER><<<gridg, 128, 0, s>>>(
+      Np, {X, m->Wb + m->wb_off[1], m->P + L.be, nullptr, m->H, m->Cat[0], 2 * HID, true, m->pos[0]});
   for (int l = 0; l < LAYERS; l++) {
-    const int aggGrid = (int)((m->N * 16LL + 255) / 256);
-    k_mean_agg<false><<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->Cat[l], 2 * HID, m->Cat[l] + HID,
-                                              2 * HID, nullptr);
-    gemm_bf16<2 * HID, HID><<<gridg, 128, 0, s>>>(Np, m->Cat[l], m->Wb + m->wb_off[2 * (l + 1) + 1], m->P + L.b[l], m->Z[l]);
+    const int aggGrid = (int)((m->N * 8LL + 255) / 256);
+    k_mean_agg<false><<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->deginv, m->Cat[l], 2 * HID,
+                                              m->Cat[l] + HID, 2 * HID, nullptr);
     bf16 *next = (l + 1 < LAYERS) ? m->Cat[l + 1] : m->H3b;
     const int ldn = (l + 1 < LAYERS) ? 2 * HID : HID;
-    k_act<<<grid1(cnt), 256, 0, s>>>(cnt, m->Z[l], m->Hf[l], m->Hf[l + 1], next, ldn);
+    gemm_bf16<2 * HID, HID, LAYER><<<gridg, 128, 0, s>>>(
+        Np, {m->Cat[l], m->Wb + m->wb_off[2 * (l + 1) + 1], m->P + L.b[l], nullptr, m->H, next, ldn, false, m->pos[l + 1]});
   }
-  gemm_bf16<HID, FOUT><<<gridg, 128, 0, s>>>(Np, m->H3b, m->Wb + m->wb_off[2 * (LAYERS + 1) + 1], m->P + L.bd, m->Y);
+  gemm_bf16<HID, FOUT, PLAIN><<<gridg, 128, 0, s>>>(
+      Np, {m->H3b, m->Wb + m->wb_off[2 * (LAYERS + 1) + 1], m->P + L.bd, m->Y, nullptr, nullptr, 0, false, nullptr});
   return cudaGetLastError() == cudaSuccess ? 0 : CFDGPU_ECUDA;
 }
 
-int wgrad(cfdgpu_mpnn *m, int w, const bf16 *A, int lda, const float *dZ)
+int wgrad(cfdgpu_mpnn *m, int w, const bf16 *A, int lda, const float *dZ, const uint64_t *pos)
 {
   cudaStream_t s = m->g.stream;
   int K, NO;
   weight_shape(w, K, NO);
-  const int rpc = wgrad_rows(m->Npad);
-  if (w == 0) k_wgrad<FIN, HID, 2, 2><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
-  else if (w <= LAYERS) k_wgrad<2 * HID, HID, 8, 4><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
-  else k_wgrad<HID, FOUT, 2, 2><<<m->nchunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, m->partial);
+  const bool wide = w > 0 && w <= LAYERS;
+  const int rpc = wgrad_rows(m->Npad, wide ? WG_CTAS<32> : WG_CTAS<4>), chunks = (m->Npad + rpc - 1) / rpc;
+  if (w == 0) k_wgrad<FIN, HID, 2, 2><<<chunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
+  else if (wide) k_wgrad<2 * HID, HID, 8, 4><<<chunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
+  else k_wgrad<HID, FOUT, 2, 2><<<chunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
   const int pairs = (K + 1) * NO;
-  k_wgrad_reduce<<<(pairs + 31) / 32, 256, 0, s>>>(m->nchunks, K, NO, m->partial, m->G + weight_off(m->L, w),
+  k_wgrad_reduce<<<(pairs + 31) / 32, 256, 0, s>>>(chunks, K, NO, m->partial, m->G + weight_off(m->L, w),
                                                      m->G + bias_off(m->L, w));
   return cudaGetLastError() == cudaSuccess ? 0 : CFDGPU_ECUDA;
 }
@@ -627,27 +698,27 @@ int backward(cfdgpu_mpnn *m, const bf16 *X, const float *T, float *loss_dev)
   cudaStream_t s = m->g.stream;
   const int Np = m->Npad;
   const int gridg = gemm_grid(Np);
-  const int64_t cnt = (int64_t)Np * HID;
   const int64_t ycnt = (int64_t)Np * FOUT;
   const float inv_cnt = 1.f / (float)std::max(1, m->g.nfree);
   const int lblocks = 148;
-  k_loss<<<lblocks, 256, 0, s>>>(ycnt, m->Y, T, m->mask, inv_cnt, m->dY, m->dYb, m->lossbuf + 1);
+  k_loss<<<lblocks, LOSS_THREADS, 0, s>>>(ycnt, m->Y, T, m->mask, inv_cnt, m->dY, m->dYb, m->lossbuf + 1);
   k_sum_partials<<<1, 32, 0, s>>>(lblocks, m->lossbuf + 1, loss_dev);
   int rc;
-  if ((rc = wgrad(m, LAYERS + 1, m->H3b, HID, m->dY))) return rc;
+  if ((rc = wgrad(m, LAYERS + 1, m->H3b, HID, m->dY, nullptr))) return rc;
   // dH = dY Wd^T  (Wd stored K x NO = 64 x 16 is the NO' x K' operand here)
-  gemm_bf16<FOUT, HID><<<gridg, 128, 0, s>>>(Np, m->dYb, m->Wb + m->wb_off[2 * (LAYERS + 1)], nullptr, m->dH);
+  gemm_bf16<FOUT, HID, PLAIN><<<gridg, 128, 0, s>>>(
+      Np, {m->dYb, m->Wb + m->wb_off[2 * (LAYERS + 1)], nullptr, m->dH, nullptr, nullptr, 0, false, nullptr});
   for (int l = LAYERS - 1; l >= 0; l--) {
-    k_relu_back<<<grid1(cnt), 256, 0, s>>>(cnt, m->dH, m->Z[l], m->dZ, m->dZb);
-    if ((rc = wgrad(m, l + 1, m->Cat[l], 2 * HID, m->dZ))) return rc;
-    // dCat = dZ W_l^T  (W_l stored K x NO = 128 x 64)
-    gemm_bf16<HID, 2 * HID><<<gridg, 128, 0, s>>>(Np, m->dZb, m->Wb + m->wb_off[2 * (l + 1)], nullptr, m->dCat);
-    k_split_dcat<<<grid1(cnt), 256, 0, s>>>(cnt, m->dCat, m->dH, m->dMs);
-    const int aggGrid = (int)((m->N * 16LL + 255) / 256);
-    k_mean_agg<true><<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->dMs, HID, nullptr, 0, m->dH);
+    // dZ = dH where the pre-activation is positive
+    if ((rc = wgrad(m, l + 1, m->Cat[l], 2 * HID, m->dH, m->pos[l + 1]))) return rc;
+    // [dH, dM] += / = dZ W_l^T  (W_l stored K x NO = 128 x 64)
+    gemm_bf16<HID, 2 * HID, BACK><<<gridg, 128, 0, s>>>(
+        Np, {nullptr, m->Wb + m->wb_off[2 * (l + 1)], nullptr, nullptr, m->dH, m->dMs, 0, false, m->pos[l + 1]});
+    const int aggGrid = (int)((m->N * 8LL + 255) / 256);
+    k_mean_agg<true><<<aggGrid, 256, 0, s>>>(m->N, m->g.rowptr, m->g.colidx, m->deginv, m->dMs, HID, nullptr, 0,
+                                             m->dH);
   }
-  k_relu_back<<<grid1(cnt), 256, 0, s>>>(cnt, m->dH, m->Ze, m->dZ, m->dZb);
-  if ((rc = wgrad(m, 0, X, FIN, m->dZ))) return rc;
+  if ((rc = wgrad(m, 0, X, FIN, m->dH, m->pos[0]))) return rc;
   return cudaGetLastError() == cudaSuccess ? 0 : CFDGPU_ECUDA;
 }
 
@@ -660,6 +731,7 @@ void use_graph(cfdgpu_mpnn *m, int k)
   m->g.stream = s;
   m->N = G.N;
   m->mask = G.mask;
+  m->deginv = G.deginv;
   m->xlo = G.xlo;
   m->xinv = G.xinv;
 }
@@ -759,23 +831,24 @@ int cfdgpu_mpnn_create(cfdgpu_handle *h, uint64_t seed, cfdgpu_mpnn **out)
     return rc;
   }
   // activations
-  if ((rc = dalloc(m, &m->X, (size_t)Np * FIN)) || (rc = dalloc(m, &m->Ze, (size_t)Np * HID)) ||
+  if ((rc = dalloc(m, &m->X, (size_t)Np * FIN)) || (rc = dalloc(m, &m->H, (size_t)Np * HID)) ||
       (rc = dalloc(m, &m->H3b, (size_t)Np * HID)) || (rc = dalloc(m, &m->Y, (size_t)Np * FOUT)))
     return rc;
   for (int l = 0; l <= LAYERS; l++)
-    if ((rc = dalloc(m, &m->Hf[l], (size_t)Np * HID))) return rc;
+    if ((rc = dalloc(m, &m->pos[l], (size_t)Np))) return rc;
   for (int l = 0; l < LAYERS; l++)
-    if ((rc = dalloc(m, &m->Cat[l], (size_t)Np * 2 * HID)) || (rc = dalloc(m, &m->Z[l], (size_t)Np * HID))) return rc;
-  if ((rc = dalloc(m, &m->dH, (size_t)Np * HID)) || (rc = dalloc(m, &m->dZ, (size_t)Np * HID)) ||
-      (rc = dalloc(m, &m->dY, (size_t)Np * FOUT)) || (rc = dalloc(m, &m->dZb, (size_t)Np * HID)) ||
+    if ((rc = dalloc(m, &m->Cat[l], (size_t)Np * 2 * HID))) return rc;
+  if ((rc = dalloc(m, &m->dH, (size_t)Np * HID)) || (rc = dalloc(m, &m->dY, (size_t)Np * FOUT)) ||
       (rc = dalloc(m, &m->dYb, (size_t)Np * FOUT)) || (rc = dalloc(m, &m->dMs, (size_t)Np * HID)) ||
-      (rc = dalloc(m, &m->dCat, (size_t)Np * 2 * HID)) || (rc = dalloc(m, &m->mask, (size_t)Np * FOUT)) ||
+      (rc = dalloc(m, &m->mask, (size_t)Np * FOUT)) || (rc = dalloc(m, &m->deginv, (size_t)m->N)) ||
       (rc = dalloc(m, &m->lossbuf, 256)))
     return rc;
-  m->nchunks = (Np + wgrad_rows(Np) - 1) / wgrad_rows(Np);
-  if ((rc = dalloc(m, &m->partial, (size_t)m->nchunks * (2 * HID + 1) * HID))) return rc;
+  // partial sums of the largest weight (the others have at most twice the chunks and an eighth of the entries)
+  const int rpc = wgrad_rows(Np, WG_CTAS<32>);
+  if ((rc = dalloc(m, &m->partial, (size_t)((Np + rpc - 1) / rpc) * (2 * HID + 1) * HID))) return rc;
   k_mask<<<(m->N + 255) / 256, 256, 0, m->g.stream>>>(m->N, m->g.ndof, m->g.fixmask, m->mask);
-  m->graphs.push_back({m->g, m->N, m->mask, m->xlo, m->xinv});
+  k_deg_inv<<<(m->N + 255) / 256, 256, 0, m->g.stream>>>(m->N, m->g.rowptr, m->deginv);
+  m->graphs.push_back({m->g, m->N, m->mask, m->deginv, m->xlo, m->xinv});
   if ((rc = refresh_bf16(m))) return rc;
   if (cudaStreamSynchronize(m->g.stream) != cudaSuccess) return CFDGPU_ECUDA;
   return 0;
@@ -871,10 +944,11 @@ int cfdgpu_mpnn_add_sample_on(cfdgpu_mpnn *m, cfdgpu_handle *h, double cond, con
   for (size_t q = 0; q < m->graphs.size(); q++)
     if (m->graphs[q].g.rowptr == gv.rowptr) k = (int)q;
   if (k < 0) {
-    cfdgpu_mpnn::Graph G{gv, gv.nNode, nullptr, {}, {}};
+    cfdgpu_mpnn::Graph G{gv, gv.nNode, nullptr, nullptr, {}, {}};
     if ((rc = graph_box(gv, G.xlo, G.xinv))) return rc;
-    if ((rc = dalloc(m, &G.mask, (size_t)m->Npad * FOUT))) return rc;
+    if ((rc = dalloc(m, &G.mask, (size_t)m->Npad * FOUT)) || (rc = dalloc(m, &G.deginv, (size_t)G.N))) return rc;
     k_mask<<<(G.N + 255) / 256, 256, 0, G0.g.stream>>>(G.N, gv.ndof, gv.fixmask, G.mask);
+    k_deg_inv<<<(G.N + 255) / 256, 256, 0, G0.g.stream>>>(G.N, gv.rowptr, G.deginv);
     m->graphs.push_back(G);
     k = (int)m->graphs.size() - 1;
   }
