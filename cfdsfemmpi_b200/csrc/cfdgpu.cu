@@ -784,7 +784,10 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
   const int ugrid = (int)std::min<int64_t>((n + UPDATE_SPAN - 1) / UPDATE_SPAN, 8 * 148);
   // Arnoldi steps j0..j0+CH-1 enqueued as one unit: directly, or (without
   // per-kernel profiling) as a CUDA graph captured once per chunk and reused
-  const int CH = h->chunk;
+  // A flexible step is an inner solve of a few hundred kernels: one at a time is
+  // enough to keep the GPU fed, and what runs on as no-ops after the last one (two
+  // microseconds a kernel) is one step, not up to 2 CH - 1.
+  const int CH = K.Z ? 1 : h->chunk;
   auto enqueue_chunk = [&](int j0) -> int {
     for (int j = j0; j < std::min(m, j0 + CH); j++) {
       int r;
