@@ -788,8 +788,14 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
   // enough to keep the GPU fed, and what runs on as no-ops after the last one (two
   // microseconds a kernel) is one step, not up to 2 CH - 1.
   const int CH = K.Z ? 1 : h->chunk;
+  // the control block as each chunk leaves it: its last kernel writes it to the
+  // host (a copy of its own costs a launch and 3 us between the graphs).  A chunk
+  // has the same place in every cycle, so its graph holds it.
+  constexpr int R = cfdgpu_handle::MAX_DEPTH + 1;
   auto enqueue_chunk = [&](int j0) -> int {
-    for (int j = j0; j < std::min(m, j0 + CH); j++) {
+    const int j1 = std::min(m, j0 + CH);
+    for (int j = j0; j < j1; j++) {
+      GmresState *snap = (j == j1 - 1) ? &h->h_gst[(j0 / CH) % R] : nullptr;
       int r;
       if ((r = arnoldi(j))) return r;
       const int pi = prof_begin(h, CFDGPU_KIND_ORTHO, (2.0 * j + 3.0) * (double)sizeof(VT) * n);
@@ -800,9 +806,9 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
         gmres_mdot<VT><<<g2, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
       }
       if (few)
-        gmres_maxpy_norm<VT, MAXPY_FEW_SPAN, 1, 8><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+        gmres_maxpy_norm<VT, MAXPY_FEW_SPAN, 1, 8><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
       else
-        gmres_maxpy_norm<VT, MAXPY_WIDE_SPAN / 2, 2, 2><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+        gmres_maxpy_norm<VT, MAXPY_WIDE_SPAN / 2, 2, 2><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
       prof_end(h, pi);
     }
     return check_launch(h, "gmres_arnoldi");
@@ -814,7 +820,7 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
     // poll the device flag `depth` chunks behind so the GPU stays fed; the
     // chunks enqueued past convergence run as no-ops
     bool stop = false;
-    const int D = h->depth, R = D + 1;
+    const int D = h->depth;
     int c = 0;
     for (int j0 = 0; j0 < m && !stop; j0 += CH, c++) {
       const int nk = std::min(m, j0 + CH) - j0;
@@ -845,7 +851,6 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
         h->launches += 2 * nk;
       }
       const int cidx = c % R;
-      CK(cudaMemcpyAsync(&h->h_gst[cidx], st, sizeof(GmresState), cudaMemcpyDeviceToHost, h->stream));
       CK(cudaEventRecord(h->evq[cidx], h->stream));
       // wait for the snapshot taken `depth` chunks ago
       if (c >= D) {

@@ -605,14 +605,16 @@ gmres_mdot_each(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, co
 // through shared memory.  One more CTA applies the stored Givens rotations to
 // column j meanwhile (a serial chain of j steps, none of which needs the norm);
 // the last CTA to arrive finishes the norm, forms the new rotation and runs the
-// convergence test (KSPGMRESUpdateHessenberg, KSPConvergedDefault).
+// convergence test (KSPGMRESUpdateHessenberg, KSPConvergedDefault).  The last step
+// of a chunk leaves a copy of the control block in pinned host memory (snap).
 //
 // Many unknowns (64 x 2 chunks): bound by reading V, 2 KB of a vector per CTA.  Few
 // unknowns (16 x 1): V comes from L2 and the time is the latency of the terms that a
 // thread adds one batch after another, so each CTA takes 16 chunks with 16
 // groups, which fills the SMs and cuts the chain to j / 128 batches.
 // With the wide form for every size and the rotations after the norm: 6.5 us at 363
-// unknowns and 50 vectors, 15.5 at 10,092 and 300; now 4.8 and 8.4.
+// unknowns and 50 vectors, 15.5 at 10,092 and 300; now 5.0 and 7.5.
+constexpr int ROT_PER = 1024 / ORTHO_THREADS;      // columns per thread of the rotations (restart <= 1000)
 constexpr int MAXPY_FEW_SPAN = 16, MAXPY_WIDE_SPAN = 128;
 // up to eight CTAs an SM in the narrow form (38,000 FP64 unknowns)
 constexpr int64_t MAXPY_FEW = (int64_t)MAXPY_FEW_SPAN * 8 * 148;
@@ -623,38 +625,66 @@ inline int maxpy_tiles(int64_t nchunk, bool few)
 }
 template <typename VT, int CL, int PER, int UN>
 __global__ void __launch_bounds__(ORTHO_THREADS, PER > 1 ? 5 : 3)
-gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresState *st, GmresArrays ga)
+gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresState *st, GmresArrays ga,
+                 GmresState *snap)
 {
-  if (!st->active || st->it != j) return;
+  if (!st->active || st->it != j) {
+    if (snap && blockIdx.x == 0 && threadIdx.x == 0) *snap = *st;
+    return;
+  }
   constexpr int E = Chunk<VT>::E, SPAN = CL * PER, GROUPS = ORTHO_THREADS / CL;
   static_assert(SPAN <= ORTHO_THREADS, "");
   __shared__ double sh[ORTHO_THREADS / 32];
   __shared__ union {
     double qs[GROUPS][E][SPAN];
-    double col[3][1024];           // column j, cosines, sines of the rotation CTA
+    struct {
+      double2 step[1024 + 16];
+      double a[1024 + 16];
+    } rot;                         // the CTA of the rotations
   } u;
   const int m = st->m;
   const int tiles = (int)gridDim.x - 1;
   if ((int)blockIdx.x == tiles) {
-    double *hc = u.col[0], *rc = u.col[1], *rs = u.col[2];
+    // a_0 = h_0, a_{q+1} = c_q h_{q+1} - s_q a_q is the chain; the products
+    // before it and the rotated entries c_q a_q + s_q h_{q+1} after it take all threads
+    double2 *st2 = u.rot.step;
+    double *a = u.rot.a;
     double *Hj = ga.H + hidx(0, j, m);
-    for (int q = threadIdx.x; q <= j; q += ORTHO_THREADS) {
-      hc[q] = Hj[q];
-      if (q < j) { rc[q] = ga.cs[q]; rs[q] = ga.sn[q]; }
+    double hq[ROT_PER], cq[ROT_PER], sq[ROT_PER];
+#pragma unroll
+    for (int i = 0; i < ROT_PER; i++) {
+      const int q = i * ORTHO_THREADS + threadIdx.x;
+      hq[i] = cq[i] = sq[i] = 0.0;
+      if (q < j) { hq[i] = Hj[q + 1]; cq[i] = ga.cs[q]; sq[i] = ga.sn[q]; st2[q] = make_double2(sq[i], cq[i] * hq[i]); }
     }
+    if (threadIdx.x == 0) a[0] = Hj[0];
     __syncthreads();
     if (threadIdx.x == 0) {
-      double a = hc[0];
-#pragma unroll 8
-      for (int q = 0; q < j; q++) {
-        const double c = rc[q], sn = rs[q], bq = hc[q + 1];
-        rc[q] = c * a + sn * bq;   // the rotated entry q
-        a = c * bq - sn * a;
+      // eight steps in registers, the next eight loaded ahead of them
+      double v = a[0];
+      double2 t[8], n[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) t[i] = st2[i];
+      for (int q = 0; q < j; q += 8) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) n[i] = st2[q + 8 + i];
+        double o[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) o[i] = v = fma(-t[i].x, v, t[i].y);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+          a[q + 1 + i] = o[i];      // past j: not read
+          t[i] = n[i];
+        }
       }
-      rc[j] = a;
     }
     __syncthreads();
-    for (int q = threadIdx.x; q <= j; q += ORTHO_THREADS) Hj[q] = rc[q];
+#pragma unroll
+    for (int i = 0; i < ROT_PER; i++) {
+      const int q = i * ORTHO_THREADS + threadIdx.x;
+      if (q < j) Hj[q] = cq[i] * a[q] + sq[i] * hq[i];
+    }
+    if (threadIdx.x == 0) Hj[j] = a[j];
   } else {
     // coefficients H(k, j) sigma_k (written by the multi-dot), read as
     // group-uniform broadcasts inside the loop
@@ -771,6 +801,7 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
       }
       st->reason = reason;
       st->active = (reason == 0 && st->it < m && st->its < st->maxit) ? 1 : 0;
+      if (snap) *snap = *st;
     }
   }
 }
