@@ -476,7 +476,7 @@ static double trsv_bytes(cfdgpu_handle *h)
 struct FactorLaunch {
   int warps, grid;
   size_t smem;
-  bool in_smem;
+  bool in_smem, wide;
 };
 static FactorLaunch factor_launch(cfdgpu_handle *h)
 {
@@ -486,7 +486,8 @@ static FactorLaunch factor_launch(cfdgpu_handle *h)
   f.in_smem = row <= PER_SM;
   f.warps = f.in_smem ? (int)std::min<size_t>(ILU_WARPS, PER_SM / row) : ILU_WARPS;
   f.smem = f.in_smem ? f.warps * row : 0;
-  const int per_sm = f.smem <= PER_SM / 2 ? 2 : 1;
+  f.wide = h->ilu.maxrow > factor_wide(h->ndof);
+  const int per_sm = !f.wide && f.smem <= PER_SM / 2 ? 2 : 1;
   const int64_t want = std::min<int64_t>(h->nNode, std::max<int64_t>(256, 2 * (int64_t)h->ilu.maxw_l));
   f.grid = (int)std::max<int64_t>(1, std::min<int64_t>((want + f.warps - 1) / f.warps, 148 * per_sm));
   return f;
@@ -498,8 +499,9 @@ static int ilu_factor_t(cfdgpu_handle *h, const T *a, T *fval, T *fdinv)
 {
   const int pi = prof_begin(h, CFDGPU_KIND_ILU, ilu_factor_bytes(h) * (sizeof(T) / 8.0));
   const FactorLaunch f = factor_launch(h);
-  CK(cudaFuncSetAttribute(ilu_factor<NB, T, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
-  ilu_factor<NB, T, T><<<f.grid, 32 * f.warps, f.smem, h->stream>>>(
+  const auto kernel = f.wide ? ilu_factor<NB, T, T, true> : ilu_factor<NB, T, T, false>;
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
+  kernel<<<f.grid, 32 * f.warps, f.smem, h->stream>>>(
       h->nNode, h->ilu.maxrow, h->rowptr, h->faslot, a, h->frow, h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder,
       h->fperm, fval, fdinv, h->iflags, h->tctl, h->frowbuf);
   prof_end(h, pi);

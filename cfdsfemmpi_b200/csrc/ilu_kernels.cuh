@@ -179,10 +179,18 @@ __device__ __forceinline__ double invert_block(const double *A, int lane, bool &
 // the complete LU of the 64 x 64 cavity (4,224 levels).  Now a pivot's inverse and
 // the blocks of its row are requested together once its flag is seen (pivots long
 // done are found by one poll of all flags), and the row's blocks that others need
-// are written and published before the rest: 3.5, 1.5, 0.25, 4.5 and 24.1 ms (FP32
+// are written and published before the rest: 3.5, 1.5, 0.25, 4.5 and 18.9 ms (FP32
 // values are rounded where they were stored before, so the factors keep their bits).
-template <int NB, typename AT, typename FT>
-__global__ void __launch_bounds__(ILU_THREADS, 2)
+//
+// UNR rounds of 32 / NB blocks are fetched at once.  Where a pivot's list takes more
+// than two fetches of two rounds (rows of over factor_wide(NB) blocks: complete LU,
+// high levels) the last pivot's fetches are on the chain one after another, and the
+// WIDE form fetches seven rounds (four of 4x4 blocks) with one CTA per SM for the
+// registers: complete LU of the 64 x 64 cavity 24.1 -> 18.9 ms.  On shorter rows
+// more rounds only cost registers (four on the O-grid: 4.5 -> 4.8 ms).
+constexpr int factor_wide(int nb) { return 4 * (32 / nb) * 2; }
+template <int NB, typename AT, typename FT, bool WIDE>
+__global__ void __launch_bounds__(ILU_THREADS, WIDE ? 1 : 2)
 ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *__restrict__ aslot,
            const AT *__restrict__ aval, const int32_t *__restrict__ fptr, const int32_t *__restrict__ fcol,
            const int32_t *__restrict__ fdiag, const int64_t *__restrict__ uoff, const uint32_t *__restrict__ umap,
@@ -191,7 +199,7 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
 {
   constexpr int BB = NB * NB;
   constexpr int PER = 32 / NB;        // blocks updated at once: lane = (block, row)
-  constexpr int UNR = 2;
+  constexpr int UNR = WIDE ? (NB == 3 ? 7 : 4) : 2;
   extern __shared__ __align__(16) double wsm[];
   __shared__ double Lsh[ILU_WARPS][BB];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
