@@ -463,31 +463,35 @@ __device__ __forceinline__ void load_row(float (&v)[T], const float *p)
 
 // weight gradient partials: part[chunk][k][o] = sum_{rows of chunk} A[r][k] dZ[r][o]
 // (A bf16 with row stride lda, dZ FP32 N x NO, taken where pos if that is given),
-// plus the bias partial in the extra row k = K.  FP32 sums, rows in order.  A thread owns TK x TO outputs, so
-// a row costs it TK + TO shared-memory words for TK TO FMAs; a warp takes four
-// k-tiles by eight o-tiles, whose 16-byte reads are broadcasts without conflicts.
-// The next 32 rows are on their way from memory while these are added.  At 64 wide
-// layers bound by the FP32 FMA rate (66 us at 275,000 rows); a thread per output,
-// two shared-memory words for each FMA, took 475; now 113,
-// and 134 with the signs applied on the way (a pass of its own for that took 47).
-// CTAs per SM: the small layers are short of loads in flight, not of FMAs
+// plus the bias partial in the extra row k = K.  FP32 sums, rows in order.  A
+// thread owns TK x TO outputs, so a row costs it TK + TO shared-memory words for
+// TK TO FMAs; a warp takes four k-tiles by eight o-tiles, whose 16-byte reads are
+// broadcasts without conflicts.  The next 32 rows are on their way from memory
+// while these are added.  The 128 x 64 layers are bound by shared-memory reads and
+// the FP32 FMA rate (66 us at 275,000 rows): a thread per output, two words for each
+// FMA, took 475; 8 x 4 tiles of 256 threads 113 (134 with the signs applied on the
+// way, whose own pass took 47); 8 x 8 tiles of 128 threads now 124.
+// CTAs per SM: three for the registers of 64 outputs a thread; the small layers are
+// short of loads in flight, not of FMAs (one thread per output 97 us, now 35 to 40)
 constexpr int WG_ROWS = 32;
-template <int OUTPUTS> constexpr int WG_CTAS = OUTPUTS == 32 ? 2 : 4;
+template <int OUTPUTS> constexpr int WG_CTAS = OUTPUTS == 64 ? 3 : 4;
 template <int K, int NO, int TK, int TO>
-__global__ void __launch_bounds__(256, WG_CTAS<TK * TO>)
+__global__ void __launch_bounds__((K / TK) * (NO / TO), WG_CTAS<TK * TO>)
 k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const float *__restrict__ dZ,
         const uint64_t *__restrict__ pos, float *__restrict__ part)
 {
-  static_assert((K / TK) * (NO / TO) == 256 && (NO / TO) % 8 == 0 && (K / TK) % 4 == 0, "tiles of 256 threads");
+  constexpr int NT = (K / TK) * (NO / TO);               // threads
+  static_assert(NT % 32 == 0 && (NO / TO) % 8 == 0 && (K / TK) % 4 == 0, "a warp is four k-tiles by eight o-tiles");
+  constexpr int OG = TO > 4 ? 4 : TO, NG = TO / OG;      // a thread's outputs: NG groups of OG, NO / NG apart
   constexpr int WO = NO / TO / 8;                        // warps along o
   constexpr int A8 = WG_ROWS * K / 8, Z4 = WG_ROWS * NO / 4;   // 16-byte pieces of a stage
-  constexpr int NA = (A8 + 255) / 256, NZ = (Z4 + 255) / 256;
+  constexpr int NA = (A8 + NT - 1) / NT, NZ = (Z4 + NT - 1) / NT;
   __shared__ __align__(16) float sa[WG_ROWS][K];
   __shared__ __align__(16) float sz[WG_ROWS][NO];
   const int r_begin = blockIdx.x * rows_per_chunk;
   const int r_end = min(Npad, r_begin + rows_per_chunk);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kt = ((warp / WO) * 4 + (lane >> 3)) * TK, ot = ((warp % WO) * 8 + (lane & 7)) * TO;
+  const int kt = ((warp / WO) * 4 + (lane >> 3)) * TK, ot = ((warp % WO) * 8 + (lane & 7)) * OG;
   float acc[TK][TO] = {}, bias[TO] = {};
   uint4 pa[NA];
   float4 pz[NZ];
@@ -496,13 +500,13 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
   auto fetch = [&](int r0) {
 #pragma unroll
     for (int i = 0; i < NA; i++) {
-      const int q = i * 256 + threadIdx.x, rr = q / (K / 8), cc = q % (K / 8) * 8;
+      const int q = i * NT + threadIdx.x, rr = q / (K / 8), cc = q % (K / 8) * 8;
       pa[i] = make_uint4(0u, 0u, 0u, 0u);
       if (q < A8 && r0 + rr < r_end) pa[i] = *reinterpret_cast<const uint4 *>(A + (int64_t)(r0 + rr) * lda + cc);
     }
 #pragma unroll
     for (int i = 0; i < NZ; i++) {
-      const int q = i * 256 + threadIdx.x, rr = q / (NO / 4), cc = q % (NO / 4) * 4;
+      const int q = i * NT + threadIdx.x, rr = q / (NO / 4), cc = q % (NO / 4) * 4;
       pz[i] = make_float4(0.f, 0.f, 0.f, 0.f);
       on[i] = 15u;
       if (q < Z4 && r0 + rr < r_end) {
@@ -515,7 +519,7 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
   for (int r0 = r_begin; r0 < r_end; r0 += WG_ROWS) {
 #pragma unroll
     for (int i = 0; i < NA; i++) {
-      const int q = i * 256 + threadIdx.x, rr = q / (K / 8), cc = q % (K / 8) * 8;
+      const int q = i * NT + threadIdx.x, rr = q / (K / 8), cc = q % (K / 8) * 8;
       if (q < A8) {
         const uint32_t w[4] = {pa[i].x, pa[i].y, pa[i].z, pa[i].w};
         float2 f[4];
@@ -527,7 +531,7 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
     }
 #pragma unroll
     for (int i = 0; i < NZ; i++) {
-      const int q = i * 256 + threadIdx.x;
+      const int q = i * NT + threadIdx.x;
       const uint32_t o = on[i];
       if (q < Z4)
         *reinterpret_cast<float4 *>(&sz[q / (NO / 4)][q % (NO / 4) * 4]) =
@@ -539,7 +543,13 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
     for (int rr = 0; rr < WG_ROWS; rr++) {
       float a[TK], z[TO];
       load_row<TK>(a, &sa[rr][kt]);
-      load_row<TO>(z, &sz[rr][ot]);
+#pragma unroll
+      for (int q = 0; q < NG; q++) {
+        float zq[OG];
+        load_row<OG>(zq, &sz[rr][ot + q * (NO / NG)]);
+#pragma unroll
+        for (int o = 0; o < OG; o++) z[q * OG + o] = zq[o];
+      }
 #pragma unroll
       for (int i = 0; i < TK; i++)
 #pragma unroll
@@ -555,10 +565,10 @@ k_wgrad(int Npad, int rows_per_chunk, const bf16 *__restrict__ A, int lda, const
 #pragma unroll
   for (int i = 0; i < TK; i++)
 #pragma unroll
-    for (int o = 0; o < TO; o++) p[(kt + i) * NO + ot + o] = acc[i][o];
+    for (int o = 0; o < TO; o++) p[(kt + i) * NO + ot + o / OG * (NO / NG) + o % OG] = acc[i][o];
   if (kt == 0) {
 #pragma unroll
-    for (int o = 0; o < TO; o++) p[K * NO + ot + o] = bias[o];
+    for (int o = 0; o < TO; o++) p[K * NO + ot + o / OG * (NO / NG) + o % OG] = bias[o];
   }
 }
 
@@ -682,9 +692,9 @@ int wgrad(cfdgpu_mpnn *m, int w, const bf16 *A, int lda, const float *dZ, const 
   int K, NO;
   weight_shape(w, K, NO);
   const bool wide = w > 0 && w <= LAYERS;
-  const int rpc = wgrad_rows(m->Npad, wide ? WG_CTAS<32> : WG_CTAS<4>), chunks = (m->Npad + rpc - 1) / rpc;
+  const int rpc = wgrad_rows(m->Npad, wide ? WG_CTAS<64> : WG_CTAS<4>), chunks = (m->Npad + rpc - 1) / rpc;
   if (w == 0) k_wgrad<FIN, HID, 2, 2><<<chunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
-  else if (wide) k_wgrad<2 * HID, HID, 8, 4><<<chunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
+  else if (wide) k_wgrad<2 * HID, HID, 8, 8><<<chunks, 128, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
   else k_wgrad<HID, FOUT, 2, 2><<<chunks, 256, 0, s>>>(m->Npad, rpc, A, lda, dZ, pos, m->partial);
   const int pairs = (K + 1) * NO;
   k_wgrad_reduce<<<(pairs + 31) / 32, 256, 0, s>>>(chunks, K, NO, m->partial, m->G + weight_off(m->L, w),
@@ -844,7 +854,7 @@ int cfdgpu_mpnn_create(cfdgpu_handle *h, uint64_t seed, cfdgpu_mpnn **out)
       (rc = dalloc(m, &m->lossbuf, 256)))
     return rc;
   // partial sums of the largest weight (the others have at most twice the chunks and an eighth of the entries)
-  const int rpc = wgrad_rows(Np, WG_CTAS<32>);
+  const int rpc = wgrad_rows(Np, WG_CTAS<64>);
   if ((rc = dalloc(m, &m->partial, (size_t)((Np + rpc - 1) / rpc) * (2 * HID + 1) * HID))) return rc;
   k_mask<<<(m->N + 255) / 256, 256, 0, m->g.stream>>>(m->N, m->g.ndof, m->g.fixmask, m->mask);
   k_deg_inv<<<(m->N + 255) / 256, 256, 0, m->g.stream>>>(m->N, m->g.rowptr, m->deginv);
