@@ -775,7 +775,7 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
   const int ntiles = (int)((nchunk + ORTHO_THREADS - 1) / ORTHO_THREADS);
   // a flexible cycle keeps to the tiled forms: it has few vectors, and its FP32
   // inner solves carry any other order of these sums on into the result
-  const bool few = nchunk <= MAXPY_FEW && !K.Z, each = nchunk <= MDOT_EACH && !K.Z;
+  const bool few = nchunk <= MAXPY_FEW && !K.Z;
   const int mtiles = maxpy_tiles(nchunk, few);
   VT *V = K.V;
   GmresState *st = K.st;
@@ -801,8 +801,11 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
       int r;
       if ((r = arnoldi(j))) return r;
       const int pi = prof_begin(h, CFDGPU_KIND_ORTHO, (2.0 * j + 3.0) * (double)sizeof(VT) * n);
-      if (each) {
-        gmres_mdot_each<VT><<<j + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      const bool each = !K.Z && mdot_each(nchunk, j + 1);
+      if (each && nchunk <= MDOT_EACH) {
+        gmres_mdot_each<VT, ORTHO_THREADS><<<j + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      } else if (each) {
+        gmres_mdot_each<VT, 1024><<<j + 1, 1024, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
       } else {
         dim3 g2(ntiles, (j + 1 + MDOT_KC - 1) / MDOT_KC);
         gmres_mdot<VT><<<g2, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);

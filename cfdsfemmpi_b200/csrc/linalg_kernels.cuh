@@ -567,30 +567,48 @@ gmres_mdot(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, const G
 
 // The same for few unknowns: one CTA per basis vector, which needs no second
 // stage over partial sums (a fence, an atomic and a dependent read, a third of
-// the multi-dot's 3.7 us at 363 unknowns; now 1.9).  Up to MDOT_EACH chunks, eight loads
-// per thread; beyond, w would be read from L2 once for every vector.
-constexpr int64_t MDOT_EACH = 8 * ORTHO_THREADS;
-template <typename VT>
-__global__ void __launch_bounds__(ORTHO_THREADS)
+// the multi-dot's 3.7 us at 363 unknowns; now 1.8).  256 threads up to MDOT_EACH
+// chunks, 1024 up to MDOT_EACH_WIDE, where a CTA's two vectors take as long as the
+// second stage; beyond, up to MDOT_EACH_FULL, only with a CTA for every SM (the
+// tiles use the whole chip for a few vectors too).  Mean over a GMRES(400) solve,
+// tiles -> this, us: 4,332 unknowns 5.1 -> 3.6, 10,092 6.1 -> 4.5, 15,987 7.4 -> 5.1,
+// 30,603 11.5 -> 7.9, 51,483 20.2 -> 14.6.
+constexpr int64_t MDOT_EACH = 8 * ORTHO_THREADS, MDOT_EACH_WIDE = 8 * 1024, MDOT_EACH_FULL = 32 * 1024;
+inline bool mdot_each(int64_t nchunk, int vectors)
+{
+  return nchunk <= MDOT_EACH_WIDE || (nchunk <= MDOT_EACH_FULL && vectors >= 148);
+}
+template <typename VT, int NT>
+__global__ void __launch_bounds__(NT)
 gmres_mdot_each(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, const GmresState *__restrict__ st,
                 GmresArrays ga)
 {
   if (!st->active || st->it != j) return;
   constexpr int E = Chunk<VT>::E;
-  __shared__ double sh[ORTHO_THREADS / 32];
+  __shared__ double sh[NT / 32];
   const int k = blockIdx.x;
   const VT *v = V + (int64_t)k * ldv, *w = V + (int64_t)(j + 1) * ldv;
   const double sigma = ga.sigma[k];
   double acc = 0.0;
-#pragma unroll 4
-  for (int64_t p = threadIdx.x; p < nchunk; p += ORTHO_THREADS) {
-    double a[E], b[E];
-    Chunk<VT>::load(v + E * p, a);
-    Chunk<VT>::load(w + E * p, b);
+  constexpr int UN = 4;
+  for (int64_t p0 = threadIdx.x; p0 < nchunk; p0 += UN * NT) {
+    double a[UN][E], b[UN][E];
 #pragma unroll
-    for (int e = 0; e < E; e++) acc = fma(a[e], b[e], acc);
+    for (int t = 0; t < UN; t++) {
+      if (p0 + t * NT < nchunk) {
+        Chunk<VT>::load(v + E * (p0 + t * NT), a[t]);
+        Chunk<VT>::load(w + E * (p0 + t * NT), b[t]);
+      }
+    }
+#pragma unroll
+    for (int t = 0; t < UN; t++) {
+      if (p0 + t * NT < nchunk) {
+#pragma unroll
+        for (int e = 0; e < E; e++) acc = fma(a[t][e], b[t][e], acc);
+      }
+    }
   }
-  acc = block_sum<ORTHO_THREADS>(acc, sh);
+  acc = block_sum<NT>(acc, sh);
   if (threadIdx.x == 0) {
     const double hkj = sigma * acc;
     ga.H[hidx(k, j, st->m)] = hkj;
