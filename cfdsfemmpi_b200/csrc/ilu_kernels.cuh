@@ -29,6 +29,7 @@
 
 #include "linalg_kernels.cuh"
 #include "trsv_plan.h"
+#include "warp_wait.h"
 
 namespace cfdgpu {
 
@@ -492,34 +493,27 @@ __device__ __forceinline__ void st_slot(uint32_t p, double v)
   asm volatile("st.volatile.shared.f64 [%0], %1;" ::"r"(p), "d"(v) : "memory");
 }
 
-// Bounded waits of ilu_trsv.  A wait gives up after TRSV_WAIT_NS, or when
-// another wait of the CTA has: ctl->error is then set and the CTA goes on with
-// what is there, so that its copies complete and it can leave.
-constexpr unsigned long long TRSV_WAIT_NS = 2000000000ull;
-struct TrsvWait {
-  volatile int *gave_up;
+// Bounded waits of ilu_trsv (warp_wait.h).  A wait gives up when its time is over
+// or another wait of the CTA has given up: ctl->error is then set and the CTA goes
+// on with what is there, so that its copies complete and it can leave.
+struct TrsvEnv {
+  volatile int *flag;
   TriCtl *ctl;
-  int it = 0;
-  unsigned long long t0 = 0;
-  // for a whole warp at once (every lane calls it)
-  __device__ __forceinline__ bool warp_goes_on()
+  __device__ __forceinline__ bool gave_up() const { return *flag != 0; }
+  __device__ __forceinline__ void give_up() const
   {
-    if ((it + 1) & 1023) { ++it; return true; }
-    return __all_sync(0xffffffffu, go_on());
+    *flag = 1;
+    atomicCAS(&ctl->error, 0u, ILU_ERR_TIMEOUT);
   }
-  __device__ __forceinline__ bool go_on()
+  __device__ __forceinline__ unsigned long long now() const
   {
-    if (++it & 1023) return true;
-    if (*gave_up) return false;
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    if (it == 1024) t0 = t;
-    if (t - t0 < TRSV_WAIT_NS) return true;
-    *gave_up = 1;
-    atomicCAS(&ctl->error, 0u, ILU_ERR_TIMEOUT);
-    return false;
+    return t;
   }
 };
+using TrsvWait = LaneWait<TrsvEnv>;
+
 // Persistent CTAs take groups of rows (TrsvPlan) in topological order.  Every
 // value a group needs has a slot in shared memory that holds the sentinel until
 // the value is known: the loader warps poll the inputs that other groups write
@@ -665,7 +659,7 @@ ilu_trsv(TrsvView P, const T *__restrict__ fval, const T *__restrict__ fdinv, co
       };
       if (tot == 0 && opens) open_gate();
       int64_t at = place(lt), nat = place(lt + LT);
-      TrsvWait wait{&s_gave_up, ctl};
+      TrsvWait wait{{&s_gave_up, ctl}};
       for (int k = lt; at >= 0;) {
         typename S::U v[UW];
         if constexpr (UW == 2) S::load2(src + at, v);
@@ -776,18 +770,17 @@ ilu_trsv(TrsvView P, const T *__restrict__ fval, const T *__restrict__ fdinv, co
         copy(s + TRSV_DEPTH - 1);     // into the stage of piece s - 1
         if (s == 0) {
           // the loader opens the gate even when its own wait runs out
-          for (TrsvWait wait{&s_gave_up, ctl}; !bar_try_wait(gate, ngone & 1u) && wait.go_on();) {}
-          __syncwarp();
+          TrsvWait wait{{&s_gave_up, ctl}};
+          wait_lanes([&] { return bar_try_wait(gate, ngone & 1u); }, wait, [] { __syncwarp(); });
         }
         // One load at a time for the input expected last; then the whole row,
         // done over in the rare case that another input was later still (the
         // check is off the path from the loads to the result).
-        TrsvWait wait{&s_gave_up, ctl};
+        TrsvWait wait{{&s_gave_up, ctl}};
         const uint32_t last = xs0 + ((uint32_t)q.m.w >> 16) * 8u + 4u;
-        while (ld_slot_hi(last) == (uint32_t)(D::bits >> 32) && wait.warp_goes_on()) {}
+        wait_lanes([&] { return ld_slot_hi(last) != (uint32_t)(D::bits >> 32); }, wait, [] { __syncwarp(); });
         double t[W], x;
-        bool again;
-        do {
+        auto row_sum = [&]() -> bool {
           U64 u[PASS][W];
           bool miss = false;
           if (q.m.z & TRSV_DIRECT) {
@@ -826,7 +819,7 @@ ilu_trsv(TrsvView P, const T *__restrict__ fval, const T *__restrict__ fdinv, co
           for (int p = 0; p < PASS; p++)
 #pragma unroll
             for (int c = 0; c < W; c++) miss |= (uint32_t)(u[p][c] >> 32) == (uint32_t)(D::bits >> 32);
-          again = __any_sync(FULL, miss);
+          const bool again = __any_sync(FULL, miss);
           double sum = t[0];
           if constexpr (W > 1) sum += t[1];
           if constexpr (W == 3) sum += t[2];
@@ -861,7 +854,9 @@ ilu_trsv(TrsvView P, const T *__restrict__ fval, const T *__restrict__ fdinv, co
               x = fma((double)q.d[0], s0, fma((double)q.d[1], s1, (double)q.d[2] * s2));
             }
           }
-        } while (again && wait.warp_goes_on());
+          return again;
+        };
+        retry_warp(row_sum, wait, [](bool v) { return (bool)__all_sync(FULL, v); });
 #pragma unroll
         for (int c = 0; c < W; c++) acc[c] = t[c];
         if (q.m.z & TRSV_LAST) {
