@@ -473,6 +473,7 @@ static double trsv_bytes(cfdgpu_handle *h)
 // CTAs: as many warps as the rows leave room for (8 at most, two CTAs per SM),
 // and no more than twice the widest dependency level holds (at least 256), since
 // warps beyond what the levels can feed only add polling traffic.
+constexpr size_t FACTOR_SMEM = 220 * 1024;    // for rows, of the 227 KB that a CTA may have
 struct FactorLaunch {
   int warps, grid;
   size_t smem;
@@ -480,7 +481,7 @@ struct FactorLaunch {
 };
 static FactorLaunch factor_launch(cfdgpu_handle *h)
 {
-  constexpr size_t PER_SM = 220 * 1024;
+  constexpr size_t PER_SM = FACTOR_SMEM;
   const size_t row = (size_t)h->ilu.maxrow * h->ndof * h->ndof * sizeof(double);
   FactorLaunch f;
   f.in_smem = row <= PER_SM;
@@ -500,7 +501,6 @@ static int ilu_factor_t(cfdgpu_handle *h, const T *a, T *fval, T *fdinv)
   const int pi = prof_begin(h, CFDGPU_KIND_ILU, ilu_factor_bytes(h) * (sizeof(T) / 8.0));
   const FactorLaunch f = factor_launch(h);
   const auto kernel = f.wide ? ilu_factor<NB, T, T, true> : ilu_factor<NB, T, T, false>;
-  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
   kernel<<<f.grid, 32 * f.warps, f.smem, h->stream>>>(
       h->nNode, h->ilu.maxrow, h->rowptr, h->faslot, a, h->frow, h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder,
       h->fperm, fval, fdinv, h->iflags, h->tctl, h->frowbuf);
@@ -516,6 +516,30 @@ static int ilu_factor_run(cfdgpu_handle *h)
                         : ilu_factor_t<3, float>(h, h->bsr32, h->fval32, h->fdinv32);
   return h->ndof == 4 ? ilu_factor_t<4, double>(h, h->bsr, h->fval, h->fdinv)
                       : ilu_factor_t<3, double>(h, h->bsr, h->fval, h->fdinv);
+}
+
+// Shared memory that the ILU kernels may be launched with.  The limit belongs to
+// the function and so to every handle and thread of the process: it is set when a
+// handle is created, always to the most that any mesh asks for, and a launch
+// leaves it alone.  (A launch that set it to its own mesh's size could lower it
+// between another thread's setting and launch.)
+template <int NB, typename T>
+static int ilu_limits(cfdgpu_handle *h)
+{
+  auto most = [](auto kernel, size_t bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  CK(most(ilu_factor<NB, T, T, true>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, false>, FACTOR_SMEM));
+  CK(most(ilu_trsv<NB, false, T>, TRSV_SMEM));
+  CK(most(ilu_trsv<NB, true, T>, TRSV_SMEM));
+  return 0;
+}
+
+static int ilu_limits(cfdgpu_handle *h)
+{
+  if (h->mixed) return h->ndof == 4 ? ilu_limits<4, float>(h) : ilu_limits<3, float>(h);
+  return h->ndof == 4 ? ilu_limits<4, double>(h) : ilu_limits<3, double>(h);
 }
 
 // Schedule of the lower or upper solve, uploaded.
@@ -544,8 +568,6 @@ static cudaError_t launch_trsv(cfdgpu_handle *h, const TrsvView &V, const T *fva
                                const GmresState *st, int j, const int *active)
 {
   const size_t smem = trsv_smem<NB, UPPER, T>(V.slots);
-  cudaError_t e = cudaFuncSetAttribute(ilu_trsv<NB, UPPER, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
   ilu_trsv<NB, UPPER, T><<<std::min(V.ngroups, 148), TRSV_THREADS, smem, h->stream>>>(V, fval, fdinv, h->fperm, r, y, z,
                                                                                     h->tctl, st, j, active);
   return cudaGetLastError();
@@ -1356,6 +1378,7 @@ int cfdgpu_create(const cfdgpu_mesh *mesh, const cfdgpu_control *ctrl, const cfd
     if ((rc = upload(h, &h->fuoff, f.uoff.data(), f.uoff.size()))) return rc;
     if ((rc = upload(h, &h->fumap, f.umap.data(), f.umap.size()))) return rc;
     if ((rc = upload(h, &h->florder, f.lorder.data(), f.lorder.size()))) return rc;
+    if ((rc = ilu_limits(h))) return rc;
     if ((rc = upload_trsv(h, false, h->plan_l)) || (rc = upload_trsv(h, true, h->plan_u))) return rc;
     if (!f.perm.empty() && (rc = upload(h, &h->fperm, f.perm.data(), f.perm.size()))) return rc;
     if (h->mixed) {
