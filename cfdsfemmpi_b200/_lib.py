@@ -21,7 +21,7 @@ EXPORTS = [
     "cfdgpu_element_matrices", "cfdgpu_set_element_state", "cfdgpu_pattern_info_get", "cfdgpu_export_pattern",
     "cfdgpu_pattern_build", "cfdgpu_ilu_pattern_build", "cfdgpu_trsv_plan_build", "cfdgpu_assemble_export", "cfdgpu_solve_export", "cfdgpu_timers", "cfdgpu_launch_count",
     "cfdgpu_set_profiling", "cfdgpu_kernel_stats", "cfdgpu_true_residual", "cfdgpu_residual_norm_noalloc",
-    "cfdgpu_ilu_export", "cfdgpu_pc_apply_export",
+    "cfdgpu_ilu_export", "cfdgpu_pc_apply_export", "cfdgpu_bcgs_scalars",
     "cfdgpu_mpnn_create", "cfdgpu_mpnn_destroy", "cfdgpu_mpnn_num_params", "cfdgpu_mpnn_get_params",
     "cfdgpu_mpnn_set_params", "cfdgpu_mpnn_set_scales", "cfdgpu_mpnn_add_sample", "cfdgpu_mpnn_num_samples",
     "cfdgpu_mpnn_set_condition", "cfdgpu_mpnn_add_sample_on",
@@ -137,6 +137,7 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     L.cfdgpu_true_residual.argtypes = [vp, vp, vp, ctypes.POINTER(ctypes.c_double)]
     L.cfdgpu_ilu_export.argtypes = [vp, ctypes.POINTER(ctypes.c_int64), vp, vp, vp, vp, vp]
     L.cfdgpu_pc_apply_export.argtypes = [vp, vp, vp]
+    L.cfdgpu_bcgs_scalars.argtypes = [ctypes.c_int64, vp, vp] + [ctypes.POINTER(dp), ctypes.POINTER(ip)] * 2
     L.cfdgpu_residual_norm_noalloc.argtypes = [ip, ip, vp, vp, vp, vp, vp, vp, vp]
     L.cfdgpu_mpnn_create.argtypes = [vp, ctypes.c_uint64, ctypes.POINTER(vp)]
     L.cfdgpu_mpnn_destroy.argtypes = [vp]
@@ -278,6 +279,21 @@ def trsv_plan_build(mesh, levels: int = 0, nblocks: int = 1, upper: bool = False
         raise CfdGpuError(rc, "triangular-solve schedule build failed")
     d["info"] = info
     return d
+
+
+def bcgs_scalars(v, w):
+    """(alpha, reason), (omega, reason) of cfdgpu_bcgs_scalars; a scalar is None where the solve would stop."""
+    L = load()
+    v, w = (np.ascontiguousarray(x, dtype=np.float64) for x in (v, w))
+    if v.shape != w.shape or v.ndim != 1:
+        raise ValueError("two vectors of one length")
+    a, o = ctypes.c_double(), ctypes.c_double()
+    ra, ro = ctypes.c_int(), ctypes.c_int()
+    rc = L.cfdgpu_bcgs_scalars(v.size, _ptr(v), _ptr(w), ctypes.byref(a), ctypes.byref(ra), ctypes.byref(o),
+                               ctypes.byref(ro))
+    if rc != 0:
+        raise CfdGpuError(rc, "BiCGStab scalars failed")
+    return (None if ra.value else a.value, ra.value), (None if ro.value else o.value, ro.value)
 
 
 class CfdGpuError(RuntimeError):

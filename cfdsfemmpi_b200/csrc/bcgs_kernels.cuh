@@ -68,20 +68,22 @@ __global__ void bcgs_setup(BcgsState *st, int maxit, double rtol, double atol, d
 // (products split exactly by FMA, Knuth's two-sum; Ogita, Rump and Oishi, 2005):
 // BiCGStab's (r, rp) and (v, rp) fall many orders below the sum of their terms'
 // magnitudes, and a plain sum can then cancel to exactly 0.0, which the
-// breakdown rule takes for an orthogonal vector.
+// breakdown rule takes for an orthogonal vector.  The transformations are exact
+// only as written, each operation rounded once: the _rn intrinsics are never
+// contracted, where a compiler may turn x * y + a into one FMA.
 struct Pair {
   double hi, lo;
 };
 
 __device__ __forceinline__ Pair pair_add(const Pair &a, const Pair &b)
 {
-  const double s = a.hi + b.hi, t = s - a.hi;
-  return {s, (a.lo + b.lo) + ((a.hi - (s - t)) + (b.hi - t))};
+  const double s = __dadd_rn(a.hi, b.hi), t = __dsub_rn(s, a.hi);
+  return {s, (a.lo + b.lo) + (__dsub_rn(a.hi, __dsub_rn(s, t)) + __dsub_rn(b.hi, t))};
 }
 
 __device__ __forceinline__ void pair_fma(Pair &acc, double x, double y)
 {
-  const double p = x * y;
+  const double p = __dmul_rn(x, y);
   acc = pair_add(acc, {p, fma(x, y, -p)});
 }
 

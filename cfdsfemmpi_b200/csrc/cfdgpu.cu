@@ -1903,6 +1903,40 @@ int cfdgpu_pc_apply_export(cfdgpu_handle *h, const double *r, double *z)
   return ilu_check(h);
 }
 
+int cfdgpu_bcgs_scalars(int64_t n, const double *v, const double *w, double *alpha, int *alpha_reason, double *omega,
+                        int *omega_reason)
+{
+  if (n <= 0 || !v || !w || !alpha || !alpha_reason || !omega || !omega_reason) return CFDGPU_EINVAL;
+  double *d = nullptr;      // v, w, partial sums
+  BcgsState *st = nullptr, s{};
+  auto run = [&](bool first) {
+    s = BcgsState{};
+    s.active = 1;
+    s.rho = 1.0;
+    if (cudaMemcpy(st, &s, sizeof(s), cudaMemcpyHostToDevice) != cudaSuccess) return false;
+    double *const dw = d + n, *const partial = d + 2 * n;
+    if (first) bcgs_alpha<double><<<bcgs_grid<double>(n), RED_THREADS>>>(n, d, dw, st, partial);
+    else bcgs_omega<double><<<bcgs_grid<double>(n), RED_THREADS>>>(n, d, dw, st, partial);
+    return cudaGetLastError() == cudaSuccess && cudaMemcpy(&s, st, sizeof(s), cudaMemcpyDeviceToHost) == cudaSuccess;
+  };
+  bool ok = cudaMalloc(&d, sizeof(double) * (2 * n + 6 * RED_BLOCKS)) == cudaSuccess &&
+            cudaMalloc(&st, sizeof(BcgsState)) == cudaSuccess &&
+            cudaMemcpy(d, v, sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess &&
+            cudaMemcpy(d + n, w, sizeof(double) * n, cudaMemcpyHostToDevice) == cudaSuccess && run(true);
+  if (ok) {
+    *alpha_reason = s.reason;
+    if (!s.reason) *alpha = s.alpha;
+    ok = run(false);
+  }
+  if (ok) {
+    *omega_reason = s.reason;
+    if (!s.reason) *omega = s.omega;
+  }
+  cudaFree(st);
+  cudaFree(d);
+  return ok ? 0 : CFDGPU_ECUDA;
+}
+
 int cfdgpu_true_residual(cfdgpu_handle *h, const double *x, const double *b, double *norm)
 {
   if (!h || !x || !b || !norm) return CFDGPU_EINVAL;

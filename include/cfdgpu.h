@@ -284,6 +284,14 @@ int cfdgpu_ilu_export(cfdgpu_handle *h, int64_t *nnzb, int32_t *rowptr, int32_t 
  * matrix (PCApply; host arrays of nNode*ndof, zero at Dirichlet dofs). */
 int cfdgpu_pc_apply_export(cfdgpu_handle *h, const double *r, double *z);
 
+/* The scalars that BiCGStab forms from two vectors (host arrays of n), by its own
+ * reductions: alpha = rho / (v, w) with rho = 1, and omega = (v, w) / (w, w).
+ * A reason is 0, or the KSP reason at which the solve would stop there (the
+ * scalar is then not written).  Replaces the VecDot calls in PETSc's KSPSolve_BCGS
+ * (SolverPetsc.cpp:253); used by tests on vectors whose products cancel. */
+int cfdgpu_bcgs_scalars(int64_t n, const double *v, const double *w, double *alpha, int *alpha_reason, double *omega,
+                        int *omega_reason);
+
 /* True (unpreconditioned) residual of the last assembled system:
  * *norm = ||b - A x||_2 with the library's deterministic reduction.  x and b
  * are host arrays of nNode*ndof doubles (zero at Dirichlet dofs). */
