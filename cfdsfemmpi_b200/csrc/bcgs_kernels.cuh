@@ -98,7 +98,8 @@ template <typename VT> using Sum = typename SumOf<VT>::type;
 template <typename VT> inline int bcgs_grid(int64_t n) { return sizeof(VT) == 4 ? RED_BLOCKS : red_grid(n); }
 __device__ __forceinline__ void sum_fma(Pair &acc, double x, double y) { pair_fma(acc, x, y); }
 __device__ __forceinline__ void sum_fma(double &acc, double x, double y) { acc = fma(x, y, acc); }
-__device__ __forceinline__ double sum_value(const Pair &v) { return v.hi + v.lo; }
+// a sum that has overflowed is what the plain sum would be: its error term is not a number
+__device__ __forceinline__ double sum_value(const Pair &v) { return isfinite(v.hi) ? v.hi + v.lo : v.hi; }
 __device__ __forceinline__ double sum_value(double v) { return v; }
 
 // sum over the CTA, valid in every thread; sh: RED_THREADS / 32 entries

@@ -65,6 +65,22 @@ def test_products_keep_their_digits_under_cancellation(n):
     assert abs(omega * ww - exact) <= bound + 5 * u * abs(exact)
 
 
+@pytest.mark.parametrize("n", [2, 5000])
+def test_overflow_and_nan_end_as_in_a_plain_sum(n):
+    """(w, w) = inf and (v, w) finite: omega = 0; infinite or undefined (v, w): KSP_DIVERGED_NANORINF; zero: breakdown."""
+    v, w = np.zeros(n), np.zeros(n)
+    v[[0, -1]], w[[0, -1]] = [1.0, 2.0], [1e200, 1e10]
+    assert _run(v, w) == ((1.0 / (1e200 + 2e10), 0), (0.0, 0))
+    assert _run(-v, w)[1] == (0.0, 0)
+    v[0] = 1e200
+    assert _run(v, w)[0] == (None, -9)
+    for bad in (np.inf, np.nan):
+        v[0], w[0] = bad, 1.0
+        assert _run(v, w)[0] == (None, -9)
+    v[[0, -1]], w[[0, -1]] = [0.0, 1.0], [1.0, 0.0]
+    assert _run(v, w) == ((None, -5), (0.0, 0))
+
+
 def _run(v, w):
     from cfdsfemmpi_b200._lib import bcgs_scalars
     return bcgs_scalars(v, w)
