@@ -19,9 +19,9 @@ EXPORTS = [
     "cfdgpu_create", "cfdgpu_destroy", "cfdgpu_last_error", "cfdgpu_step", "cfdgpu_get_solution",
     "cfdgpu_set_solution", "cfdgpu_device_solution", "cfdgpu_stream", "cfdgpu_set_history", "cfdgpu_get_history",
     "cfdgpu_element_matrices", "cfdgpu_set_element_state", "cfdgpu_pattern_info_get", "cfdgpu_export_pattern",
-    "cfdgpu_pattern_build", "cfdgpu_ilu_pattern_build", "cfdgpu_trsv_plan_build", "cfdgpu_assemble_export", "cfdgpu_solve_export", "cfdgpu_timers", "cfdgpu_launch_count",
+    "cfdgpu_pattern_build", "cfdgpu_ilu_pattern_build", "cfdgpu_trsv_plan_build", "cfdgpu_trsv_by_chains", "cfdgpu_assemble_export", "cfdgpu_solve_export", "cfdgpu_timers", "cfdgpu_launch_count",
     "cfdgpu_set_profiling", "cfdgpu_kernel_stats", "cfdgpu_true_residual", "cfdgpu_residual_norm_noalloc",
-    "cfdgpu_ilu_export", "cfdgpu_pc_apply_export", "cfdgpu_bcgs_scalars",
+    "cfdgpu_ilu_export", "cfdgpu_pc_apply_export", "cfdgpu_ilu32_apply_export", "cfdgpu_bcgs_scalars",
     "cfdgpu_mpnn_create", "cfdgpu_mpnn_destroy", "cfdgpu_mpnn_num_params", "cfdgpu_mpnn_get_params",
     "cfdgpu_mpnn_set_params", "cfdgpu_mpnn_set_scales", "cfdgpu_mpnn_add_sample", "cfdgpu_mpnn_num_samples",
     "cfdgpu_mpnn_set_condition", "cfdgpu_mpnn_add_sample_on",
@@ -131,12 +131,14 @@ def load(build_if_missing: bool = True) -> ctypes.CDLL:
     L.cfdgpu_pattern_build.argtypes = [ctypes.POINTER(Mesh), ctypes.POINTER(PatternInfo)] + [vp] * 8
     L.cfdgpu_ilu_pattern_build.argtypes = [ctypes.POINTER(Mesh), ip, ip, ctypes.POINTER(IluInfo)] + [vp] * 9
     L.cfdgpu_trsv_plan_build.argtypes = [ctypes.POINTER(Mesh), ip, ip, ip, ctypes.POINTER(TrsvInfo)] + [vp] * 5
+    L.cfdgpu_trsv_by_chains.argtypes = [ctypes.POINTER(Mesh), ip, ip, ip, ctypes.POINTER(ip)]
     L.cfdgpu_assemble_export.argtypes = [vp, ip, vp, vp]
     L.cfdgpu_solve_export.argtypes = [vp, vp, vp, ctypes.POINTER(ip), ctypes.POINTER(ip)]
     L.cfdgpu_timers.argtypes = [vp, vp]
     L.cfdgpu_true_residual.argtypes = [vp, vp, vp, ctypes.POINTER(ctypes.c_double)]
     L.cfdgpu_ilu_export.argtypes = [vp, ctypes.POINTER(ctypes.c_int64), vp, vp, vp, vp, vp]
     L.cfdgpu_pc_apply_export.argtypes = [vp, vp, vp]
+    L.cfdgpu_ilu32_apply_export.argtypes = [vp, vp, vp, vp, vp]
     L.cfdgpu_bcgs_scalars.argtypes = [ctypes.c_int64, vp, vp] + [ctypes.POINTER(dp), ctypes.POINTER(ip)] * 2
     L.cfdgpu_residual_norm_noalloc.argtypes = [ip, ip, vp, vp, vp, vp, vp, vp, vp]
     L.cfdgpu_mpnn_create.argtypes = [vp, ctypes.c_uint64, ctypes.POINTER(vp)]
@@ -279,6 +281,17 @@ def trsv_plan_build(mesh, levels: int = 0, nblocks: int = 1, upper: bool = False
         raise CfdGpuError(rc, "triangular-solve schedule build failed")
     d["info"] = info
     return d
+
+
+def trsv_by_chains(mesh, levels: int = 0, nblocks: int = 1, upper: bool = False) -> bool:
+    """Whether a handle solves this triangle by chains of rows (cfdgpu_trsv_by_chains); needs no GPU."""
+    L = load()
+    m, keep = _mesh_struct(mesh)
+    v = ctypes.c_int()
+    rc = L.cfdgpu_trsv_by_chains(ctypes.byref(m), levels, nblocks, int(upper), ctypes.byref(v))
+    if rc != 0:
+        raise CfdGpuError(rc, "triangular-solve schedule build failed")
+    return bool(v.value)
 
 
 def bcgs_scalars(v, w):
@@ -480,6 +493,16 @@ class Handle:
         z = np.zeros(self.n)
         self._check(self._L.cfdgpu_pc_apply_export(self.h, _ptr(rr), _ptr(z)))
         return z
+
+    def ilu32_apply(self, r: np.ndarray):
+        """z = (L U)^-1 r with the FP32 factors of a mixed handle, and the factors: (z, vals, dinv)."""
+        rr = np.ascontiguousarray(r, dtype=np.float32)
+        f = self.ilu_factors(values=False)
+        nb = self.ndof
+        z = np.zeros(self.n, np.float32)
+        vals, dinv = np.zeros((f["colidx"].size, nb, nb), np.float32), np.zeros((self.nNode, nb, nb), np.float32)
+        self._check(self._L.cfdgpu_ilu32_apply_export(self.h, _ptr(rr), _ptr(z), _ptr(vals), _ptr(dinv)))
+        return z, vals, dinv
 
     def true_residual(self, x: np.ndarray, b: np.ndarray) -> float:
         xx = np.ascontiguousarray(x, dtype=np.float64)

@@ -17,7 +17,7 @@ struct Run {
 
 }  // namespace
 
-void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p)
+void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p, bool choose)
 {
   p = TrsvPlan();
   const int cap = trsv_cap(nb), nslots = trsv_slots(nb), max_slots = trsv_max_slots(nb);
@@ -29,12 +29,17 @@ void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p)
 
   // dependency level of every row (rows come to be solved in about this order)
   std::vector<int32_t> lev(n, 0);
+  int levels = 0;
+  int64_t off = 0;
   for (int s = 0; s < n; s++) {
     const int i = upper ? n - 1 - s : s;
     int d = 0;
     for (int q = q0(i); q < q1(i); q++) d = std::max(d, lev[f.colidx[q]] + 1);
     lev[i] = d;
+    levels = std::max(levels, d + 1);
+    off += q1(i) - q0(i);
   }
+  const double at_once = (double)n / std::max(levels, 1);
 
   // segments: runs of consecutive chains (in solve order) each depending on
   // the one before; strands: chains of a segment cut only by the length limit
@@ -106,7 +111,11 @@ void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p)
     self(self, r0, m, cyc);
     self(self, m, r1, cyc);
   };
-  if ((int64_t)strands.size() * TRSV_SHORT_STRAND > n) {
+  int64_t in_turn = 0;            // rows in groups whose rows go to all warps in turn
+  const bool level_order = (int64_t)strands.size() * TRSV_SHORT_STRAND > n;
+  if (level_order) {
+    p.chains = at_once >= TRSV_LEVEL_P || (double)off / levels >= TRSV_LEVEL_BLOCKS;
+    if (p.chains && choose) return;
     // level order: groups small enough that every SM has some
     const std::vector<int32_t> &by_level = upper ? f.uorder : f.lorder;
     const int step = std::max(16, std::min(TRSV_LEVEL_ROWS, n / (2 * 148)));
@@ -134,6 +143,7 @@ void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p)
       if (blocks > (int64_t)len * TRSV_CYCLIC_BLOCKS) {
         // half the slots for the group's own rows, the other half for its inputs
         const int step = std::max(1, max_slots / 2);
+        in_turn += len;
         for (int x = 0; x < len; x += step)
           cut(cut, rows.data() + sp[s0] + x, rows.data() + sp[s0] + std::min(len, x + step), true);
         continue;
@@ -144,6 +154,13 @@ void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p)
     }
   }
   const int ng = (int)cyclic.size();
+  if (!level_order) {
+    if (2 * in_turn > n)
+      p.chains = at_once >= TRSV_CYCLIC_P && n >= (int64_t)TRSV_CYCLIC_ROWS * ng;
+    else
+      p.chains = TRSV_GROUP_US * ng / 148 > levels * (TRSV_LEVEL_US + trsv_block_us(nb) * (double)off / n);
+    if (p.chains && choose) return;
+  }
 
   // order of the groups: topological, lowest level first
   std::vector<int32_t> group_of(n), order;
@@ -223,7 +240,7 @@ void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p)
         p.wptr.push_back((int32_t)p.pieces.size());
       }
     } else {
-      // a strand's rows to a pair of warps in turn
+      // a strand's rows to four warps in turn
       constexpr int PER = TRSV_WARPS / TRSV_STRANDS;
       int w = 0;
       for (int x0 = 0, x1; x0 < rows; x0 = x1) {

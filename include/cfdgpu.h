@@ -257,6 +257,10 @@ typedef struct cfdgpu_trsv_info {
 int cfdgpu_trsv_plan_build(const cfdgpu_mesh *mesh, int levels, int nblocks, int upper, cfdgpu_trsv_info *info,
                            int32_t *groups, int32_t *wptr, int32_t *pieces, uint32_t *desc, int32_t *ext);
 
+/* Host-only: *by_chains = 1 if a handle solves this triangle by chains of rows
+ * (the arrays of cfdgpu_ilu_pattern_build) and not by the groups above. */
+int cfdgpu_trsv_by_chains(const cfdgpu_mesh *mesh, int levels, int nblocks, int upper, int *by_chains);
+
 /* Assemble (iteration-0 semantics when iter == 0: lifting included) at the
  * current state and copy the BSR values (nnzb*ndof*ndof, FP64, block
  * row-major) and the RHS (nNode*ndof) to host.  Uses the td[] of the last
@@ -283,6 +287,11 @@ int cfdgpu_ilu_export(cfdgpu_handle *h, int64_t *nnzb, int32_t *rowptr, int32_t 
 /* z = M^-1 r with the handle's preconditioner, built from the last assembled
  * matrix (PCApply; host arrays of nNode*ndof, zero at Dirichlet dofs). */
 int cfdgpu_pc_apply_export(cfdgpu_handle *h, const double *r, double *z);
+
+/* The same of a mixed-precision handle with block ILU: z = (L U)^-1 r on FP32
+ * vectors (host arrays of nNode*ndof), and the FP32 factors that it used, in the
+ * layout of cfdgpu_ilu_export (vals, dinv; either may be NULL). */
+int cfdgpu_ilu32_apply_export(cfdgpu_handle *h, const float *r, float *z, float *vals, float *dinv);
 
 /* The scalars that BiCGStab forms from two vectors (host arrays of n), by its own
  * reductions: alpha = rho / (v, w) with rho = 1, and omega = (v, w) / (w, w).
