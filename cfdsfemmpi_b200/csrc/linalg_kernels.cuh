@@ -634,8 +634,12 @@ gmres_mdot_each(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, co
 // unknowns and 50 vectors, 15.5 at 10,092 and 300; now 5.0 and 7.5.
 constexpr int ROT_PER = 1024 / ORTHO_THREADS;      // columns per thread of the rotations (restart <= 1000)
 constexpr int MAXPY_FEW_SPAN = 16, MAXPY_WIDE_SPAN = 128;
-// up to eight CTAs an SM in the narrow form (38,000 FP64 unknowns)
-constexpr int64_t MAXPY_FEW = (int64_t)MAXPY_FEW_SPAN * 8 * 148;
+// The narrow form pays while its CTAs, three an SM, are resident at once (14,208 FP64
+// unknowns): a step of the hex8 cavity with 19,652 and 37,044 unknowns took 9.6 and
+// 13.6 ms with it and 8.8 and 11.0 with the wide one, quad4 with 30,603 25.8 and 23.2;
+// with 12,675 5.9 and 6.9 the other way.
+constexpr int MAXPY_WAVE = 3 * 148;
+constexpr int64_t MAXPY_FEW = (int64_t)MAXPY_FEW_SPAN * MAXPY_WAVE;
 inline int maxpy_tiles(int64_t nchunk, bool few)
 {
   const int span = few ? MAXPY_FEW_SPAN : MAXPY_WIDE_SPAN;
