@@ -704,10 +704,9 @@ static int spmv_pc(cfdgpu_handle *h, int mode, const double *x, const double *b,
     }
 #undef SPMV4
   } else {
-    const int grid = (int)((h->nNode * 32LL + 255) / 256);
-#define SPMV3(MO, PCV)                                                                                         \
-  bsr3_spmv<MO, PCV, double, double><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr, x, b, \
-                                                                  h->dinv, h->binv, y, st, j, xscale, active)
+#define SPMV3(MO, PCV)                                                                                              \
+  launch_bsr3<MO, PCV, double, double>(h->stream, h->nNode, h->rowptr, h->colidx, h->bsr, x, b, h->dinv, h->binv, y, \
+                                       st, j, xscale, active)
     if (mode == 0) {
       if (pc == 0) SPMV3(0, 0); else if (pc == 1) SPMV3(0, 1); else SPMV3(0, 2);
     } else {
@@ -742,13 +741,11 @@ static int spmv32_pc(cfdgpu_handle *h, const float *x, float *y, const GmresStat
     else
       bsr4_spmv_f32<2><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, h->dinv32, h->binv32, y, st, j, xscale, active);
   } else {
-    const int grid = (int)((h->nNode * 32LL + 255) / 256);
-    if (pc == 0)
-      bsr3_spmv<0, 0, float, float><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, y, st, j, xscale, active);
-    else if (pc == 1)
-      bsr3_spmv<0, 1, float, float><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, y, st, j, xscale, active);
-    else
-      bsr3_spmv<0, 2, float, float><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, y, st, j, xscale, active);
+#define SPMV3(PCV)                                                                                                   \
+  launch_bsr3<0, PCV, float, float>(h->stream, h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, \
+                                    y, st, j, xscale, active)
+    if (pc == 0) SPMV3(0); else if (pc == 1) SPMV3(1); else SPMV3(2);
+#undef SPMV3
   }
   prof_end(h, pi);
   LAUNCHED(h);
@@ -2126,9 +2123,8 @@ extern "C" int cfdgpu_residual_norm_noalloc(int nNode, int ndof, const int32_t *
     bsr4_spmv<1, 0, double><<<grid, 256, 0, s>>>(nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr, r,
                                                 nullptr, 0, nullptr);
   } else {
-    const int grid = (int)((nNode * 32LL + 255) / 256);
-    bsr3_spmv<1, 0, double, double><<<grid, 256, 0, s>>>(nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr,
-                                                         r, nullptr, 0, nullptr);
+    launch_bsr3<1, 0, double, double>(s, nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr, r, nullptr, 0,
+                                      nullptr);
   }
   if (cudaGetLastError() != cudaSuccess) return CFDGPU_ECUDA;
   norm2_kernel<<<RED_BLOCKS, RED_THREADS, 0, s>>>(n, r, partial, counter, d_norm);

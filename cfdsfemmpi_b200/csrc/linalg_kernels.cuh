@@ -219,6 +219,12 @@ bsr4_spmv_f32(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__re
 // blocks one after another and with point-block Jacobi went over the whole node
 // three times, took 5.7 us (Jacobi, 363 unknowns) and 7.9 (point-block, 10,092);
 // now 2.4 and 3.6.  ST: type of the vectors and of the sums; MT: of the blocks.
+// With more rows than fill the chip it is bound by its instructions (three lanes of
+// a warp add), and a thread per scalar row (bsr3_spmv_rows) is the better one from
+// BSR3_WARPS rows on.  Between events (about 5 us more), warps / threads, Jacobi and
+// point-block: 10,201 nodes 11.0 / 11.9 and 11.6 / 13.0 us, 25,921 16.8 / 12.8 and
+// 18.8 / 17.2, 160,801 72 / 36 and 81 / 67.
+constexpr int64_t BSR3_WARPS = 148 * 96;
 template <int MODE, int PC, typename MT, typename ST>
 __global__ void __launch_bounds__(256)
 bsr3_spmv(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
@@ -276,6 +282,58 @@ bsr3_spmv(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__restri
     v = fma(pc[2], v2, fma(pc[1], v1, pc[0] * v0));
   }
   if (lane < 3) y[r] = v;
+}
+
+// The same with one thread per scalar row, the same sums in the same order.  With
+// point-block Jacobi a thread adds all three rows of its node.
+template <int MODE, int PC, typename MT, typename ST>
+__global__ void __launch_bounds__(256)
+bsr3_spmv_rows(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__restrict__ colidx,
+               const MT *__restrict__ val, const ST *__restrict__ x, const ST *__restrict__ b,
+               const ST *__restrict__ dinv, const ST *__restrict__ binv, ST *__restrict__ y,
+               const GmresState *__restrict__ st, int j, const double *__restrict__ xscale,
+               const int *__restrict__ active = nullptr)
+{
+  if (st && (!st->active || st->it != j)) return;
+  if (active && !active[0]) return;
+  const ST xs = xscale ? (ST)xscale[0] : (ST)1;
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t node = t / 3;
+  const int row = (int)(t % 3);
+  if (node >= nrows) return;
+  const int kb0 = rowptr[node], kb1 = rowptr[node + 1];
+  auto sum = [&](int r) {
+    ST acc = 0;
+    for (int kb = kb0; kb < kb1; kb++) {
+      const int64_t c = (int64_t)colidx[kb] * 3;
+      const MT *a = val + (int64_t)kb * 9 + r * 3;
+#pragma unroll
+      for (int q = 0; q < 3; q++) acc = fma((ST)a[q], x[c + q], acc);
+    }
+    return (MODE == 1) ? b[node * 3 + r] - xs * acc : xs * acc;
+  };
+  ST v;
+  if constexpr (PC == 2) {
+    const ST v0 = sum(0), v1 = sum(1), v2 = sum(2);
+    const ST *m = binv + node * 9 + row * 3;
+    v = fma(m[2], v2, fma(m[1], v1, m[0] * v0));
+  } else {
+    v = sum(row);
+    if (PC == 1) v *= dinv[t];
+  }
+  y[t] = v;
+}
+
+// The launch of either.
+template <int MODE, int PC, typename MT, typename ST>
+inline void launch_bsr3(cudaStream_t s, int nrows, const int32_t *rowptr, const int32_t *colidx,
+                        const MT *val, const ST *x, const ST *b, const ST *dinv, const ST *binv, ST *y,
+                        const GmresState *st, int j, const double *xscale, const int *active = nullptr)
+{
+  if (nrows <= BSR3_WARPS)
+    bsr3_spmv<MODE, PC, MT, ST><<<(int)((nrows * 32LL + 255) / 256), 256, 0, s>>>(nrows, rowptr, colidx, val, x, b, dinv, binv, y, st, j, xscale, active);
+  else
+    bsr3_spmv_rows<MODE, PC, MT, ST><<<(int)((nrows * 3LL + 255) / 256), 256, 0, s>>>(nrows, rowptr, colidx, val, x, b, dinv, binv, y, st, j, xscale, active);
 }
 
 // z = M^-1 r (stand-alone preconditioner application)

@@ -14,6 +14,7 @@ CASES = [
     # mesh, pc, restart, iterations, time step (a long one from rest converges slowly, so that late vectors count)
     ("quad", 36, "pbjacobi", 320, 257, 10.0), ("quad", 36, "jacobi", 400, 300, 10.0), ("hex", 16, "jacobi", 200, 160, 0.1),
     ("quad", 66, "pbjacobi", 60, 50, 0.1), ("quad", 68, "jacobi", 60, 50, 0.1),
+    ("quad", 118, "pbjacobi", 30, 20, 0.1), ("quad", 119, "pbjacobi", 30, 20, 0.1), ("quad", 119, "jacobi", 30, 20, 0.1),
 ]
 
 
