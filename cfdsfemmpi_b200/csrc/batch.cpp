@@ -104,8 +104,9 @@ void worker_main(cfdgpu_batch *b, int id)
 
 int apply_schedule(cfdgpu_batch *b, cfdgpu_batch::Sched s)
 {
+  const int sharers = std::min(s.concurrency, (int)b->h.size());
   for (auto *h : b->h) {
-    const int rc = cfdgpu::set_host_schedule(h, true, s.chunk, s.depth);
+    const int rc = cfdgpu::set_host_schedule(h, true, s.chunk, s.depth, sharers);
     if (rc) return rc;
   }
   b->cur = s;

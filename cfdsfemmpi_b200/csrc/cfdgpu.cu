@@ -99,6 +99,7 @@ struct cfdgpu_handle {
   bool blocking = false;   // host waits sleep (cudaEventBlockingSync) instead of spinning
   int chunk = 8;           // Arnoldi steps enqueued (and replayed as one graph) between host polls
   int depth = 1;           // chunks enqueued beyond the one whose state the host waits for
+  int sharers = 1;         // instances (this one included) that a batch steps at once
   double newton_target = 1e-8;   // this step's Newton stopping residual (absolute, and relative when asked)
   // learned initial guess
   cfdgpu_mpnn *guess = nullptr;
@@ -705,8 +706,8 @@ static int spmv_pc(cfdgpu_handle *h, int mode, const double *x, const double *b,
 #undef SPMV4
   } else {
 #define SPMV3(MO, PCV)                                                                                              \
-  launch_bsr3<MO, PCV, double, double>(h->stream, h->nNode, h->rowptr, h->colidx, h->bsr, x, b, h->dinv, h->binv, y, \
-                                       st, j, xscale, active)
+  launch_bsr3<MO, PCV, double, double>(h->stream, h->sharers, h->nNode, h->rowptr, h->colidx, h->bsr, x, b, h->dinv, \
+                                       h->binv, y, st, j, xscale, active)
     if (mode == 0) {
       if (pc == 0) SPMV3(0, 0); else if (pc == 1) SPMV3(0, 1); else SPMV3(0, 2);
     } else {
@@ -741,9 +742,9 @@ static int spmv32_pc(cfdgpu_handle *h, const float *x, float *y, const GmresStat
     else
       bsr4_spmv_f32<2><<<grid, 256, 0, h->stream>>>(h->nNode, h->rowptr, h->colidx, h->bsr32, x, h->dinv32, h->binv32, y, st, j, xscale, active);
   } else {
-#define SPMV3(PCV)                                                                                                   \
-  launch_bsr3<0, PCV, float, float>(h->stream, h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, h->dinv32, h->binv32, \
-                                    y, st, j, xscale, active)
+#define SPMV3(PCV)                                                                                            \
+  launch_bsr3<0, PCV, float, float>(h->stream, h->sharers, h->nNode, h->rowptr, h->colidx, h->bsr32, x, nullptr, \
+                                    h->dinv32, h->binv32, y, st, j, xscale, active)
     if (pc == 0) SPMV3(0); else if (pc == 1) SPMV3(1); else SPMV3(2);
 #undef SPMV3
   }
@@ -815,7 +816,8 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
   // a flexible cycle keeps to the tiled forms: it has few vectors, and its FP32
   // inner solves carry any other order of these sums on into the result
   const bool few = nchunk <= MAXPY_FEW && !K.Z;
-  const int mtiles = maxpy_tiles(nchunk, few);
+  const bool narrow = few && maxpy_narrow(nchunk, h->sharers);
+  const int mtiles = maxpy_tiles(nchunk, narrow);
   VT *V = K.V;
   GmresState *st = K.st;
   int rc;
@@ -831,28 +833,38 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
   const int CH = K.Z ? 1 : h->chunk;
   // the control block as each chunk leaves it: its last kernel writes it to the
   // host (a copy of its own costs a launch and 3 us between the graphs).  A chunk
-  // has the same place in every cycle, so its graph holds it.
+  // has the same place in every cycle, so its graph holds it.  Where instances share
+  // the chip, a copy: the kernel would hold its SM until the write has crossed the
+  // bus (64 instances of 12,675 unknowns 144 ms a step instead of 118, 32 of 8,788
+  // 27.5 instead of 24.3), and the gap in one stream is filled by others.
   constexpr int R = cfdgpu_handle::MAX_DEPTH + 1;
   auto enqueue_chunk = [&](int j0) -> int {
     const int j1 = std::min(m, j0 + CH);
     for (int j = j0; j < j1; j++) {
-      GmresState *snap = (j == j1 - 1) ? &h->h_gst[(j0 / CH) % R] : nullptr;
+      GmresState *snap = (j == j1 - 1 && h->sharers == 1) ? &h->h_gst[(j0 / CH) % R] : nullptr;
       int r;
       if ((r = arnoldi(j))) return r;
       const int pi = prof_begin(h, CFDGPU_KIND_ORTHO, (2.0 * j + 3.0) * (double)sizeof(VT) * n);
       const bool each = !K.Z && mdot_each(nchunk, j + 1);
-      if (each && nchunk <= MDOT_EACH) {
-        gmres_mdot_each<VT, ORTHO_THREADS><<<j + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
-      } else if (each) {
-        gmres_mdot_each<VT, 1024><<<j + 1, 1024, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+      if (each) {
+        const int nt = nchunk <= MDOT_EACH ? ORTHO_THREADS : 1024;
+        if (mdot_shared(nt, j + 1, h->sharers)) {
+          const auto kernel = nt == 1024 ? gmres_mdot_shared<VT, 1024> : gmres_mdot_shared<VT, ORTHO_THREADS>;
+          kernel<<<(j + MDOT_SHARED) / MDOT_SHARED, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+        } else {
+          const auto kernel = nt == 1024 ? gmres_mdot_each<VT, 1024> : gmres_mdot_each<VT, ORTHO_THREADS>;
+          kernel<<<j + 1, nt, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
+        }
       } else {
         dim3 g2(ntiles, (j + 1 + MDOT_KC - 1) / MDOT_KC);
         gmres_mdot<VT><<<g2, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga);
       }
-      if (few)
-        gmres_maxpy_norm<VT, MAXPY_FEW_SPAN, 1, 8><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
+      if (narrow)
+        gmres_maxpy_norm<VT, MAXPY_FEW_SPAN, 1, 8, 1><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
+      else if (few)
+        gmres_maxpy_norm<VT, MAXPY_WIDE_SPAN, 1, 1, 8><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
       else
-        gmres_maxpy_norm<VT, MAXPY_WIDE_SPAN / 2, 2, 2><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
+        gmres_maxpy_norm<VT, MAXPY_WIDE_SPAN / 2, 2, 2, 1><<<mtiles + 1, ORTHO_THREADS, 0, h->stream>>>(nchunk, V, ldv, j, st, K.ga, snap);
       prof_end(h, pi);
     }
     return check_launch(h, "gmres_arnoldi");
@@ -895,6 +907,8 @@ static int gmres_run(cfdgpu_handle *h, Krylov<VT> &K, double *x, int max_it, dou
         h->launches += 2 * nk;
       }
       const int cidx = c % R;
+      if (h->sharers > 1)
+        CK(cudaMemcpyAsync(&h->h_gst[cidx], st, sizeof(GmresState), cudaMemcpyDeviceToHost, h->stream));
       CK(cudaEventRecord(h->evq[cidx], h->stream));
       // wait for the snapshot taken `depth` chunks ago
       if (c >= D) {
@@ -1180,9 +1194,9 @@ static int check_negjac(cfdgpu_handle *h)
 
 namespace cfdgpu {
 
-int set_host_schedule(cfdgpu_handle *h, bool blocking, int chunk, int depth)
+int set_host_schedule(cfdgpu_handle *h, bool blocking, int chunk, int depth, int sharers)
 {
-  if (!h || chunk < 1 || chunk > 64 || depth < 1 || depth > cfdgpu_handle::MAX_DEPTH) return CFDGPU_EINVAL;
+  if (!h || sharers < 1 || chunk < 1 || chunk > 64 || depth < 1 || depth > cfdgpu_handle::MAX_DEPTH) return CFDGPU_EINVAL;
   if (blocking != h->blocking) {
     constexpr int NE = cfdgpu_handle::MAX_DEPTH + 2;
     cudaEvent_t e[NE] = {};
@@ -1196,13 +1210,14 @@ int set_host_schedule(cfdgpu_handle *h, bool blocking, int chunk, int depth)
     h->blocking = blocking;
   }
   h->depth = depth;
-  if (chunk != h->chunk) {
-    // the cached Arnoldi graphs hold chunk-length pieces of the cycle
+  if (chunk != h->chunk || sharers != h->sharers) {
+    // the cached Arnoldi graphs hold chunk-length pieces of the cycle, of kernels chosen by the sharers
     CK(cudaStreamSynchronize(h->stream));
     for (auto &g : h->graphs64) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     for (auto &g : h->graphs32) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     for (auto &g : h->graphs_bcgs) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     h->chunk = chunk;
+    h->sharers = sharers;
   }
   return 0;
 }
@@ -2123,7 +2138,7 @@ extern "C" int cfdgpu_residual_norm_noalloc(int nNode, int ndof, const int32_t *
     bsr4_spmv<1, 0, double><<<grid, 256, 0, s>>>(nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr, r,
                                                 nullptr, 0, nullptr);
   } else {
-    launch_bsr3<1, 0, double, double>(s, nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr, r, nullptr, 0,
+    launch_bsr3<1, 0, double, double>(s, 1, nNode, d_rowptr, d_colidx, d_val, d_x, d_b, nullptr, nullptr, r, nullptr, 0,
                                       nullptr);
   }
   if (cudaGetLastError() != cudaSuccess) return CFDGPU_ECUDA;

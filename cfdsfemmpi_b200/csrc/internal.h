@@ -22,9 +22,10 @@ int handle_graph(cfdgpu_handle *h, GraphView *out);
 
 // host-side scheduling of a handle's step: blocking (sleeping) host waits,
 // the number of Arnoldi steps per graph chunk (1..64) and the number of
-// chunks in flight beyond the one the host waits for (1..8); results do not
-// depend on any of them (Arnoldi kernels after convergence are no-ops)
-int set_host_schedule(cfdgpu_handle *h, bool blocking, int chunk, int depth);
+// chunks in flight beyond the one the host waits for (1..8), and the number of
+// instances stepped at once; results do not depend on any of them (Arnoldi
+// kernels after convergence are no-ops, kernels for a shared chip keep the order of sums)
+int set_host_schedule(cfdgpu_handle *h, bool blocking, int chunk, int depth, int sharers);
 
 // replace the handle's stream by a non-blocking stream of the given
 // priority (lower value = higher priority); cached Arnoldi graphs follow the

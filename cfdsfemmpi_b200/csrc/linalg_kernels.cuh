@@ -221,9 +221,10 @@ bsr4_spmv_f32(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__re
 // now 2.4 and 3.6.  ST: type of the vectors and of the sums; MT: of the blocks.
 // With more rows than fill the chip it is bound by its instructions (three lanes of
 // a warp add), and a thread per scalar row (bsr3_spmv_rows) is the better one from
-// BSR3_WARPS rows on.  Between events (about 5 us more), warps / threads, Jacobi and
-// point-block: 10,201 nodes 11.0 / 11.9 and 11.6 / 13.0 us, 25,921 16.8 / 12.8 and
-// 18.8 / 17.2, 160,801 72 / 36 and 81 / 67.
+// BSR3_WARPS rows on, those of the instances that share the chip taken together.
+// Between events (about 5 us more), warps / threads, Jacobi and point-block:
+// 10,201 nodes 11.0 / 11.9 and 11.6 / 13.0 us, 25,921 16.8 / 12.8 and 18.8 / 17.2,
+// 160,801 72 / 36 and 81 / 67.  64 instances of 4,225 nodes: 127 / 118 ms a step.
 constexpr int64_t BSR3_WARPS = 148 * 96;
 template <int MODE, int PC, typename MT, typename ST>
 __global__ void __launch_bounds__(256)
@@ -326,11 +327,11 @@ bsr3_spmv_rows(int nrows, const int32_t *__restrict__ rowptr, const int32_t *__r
 
 // The launch of either.
 template <int MODE, int PC, typename MT, typename ST>
-inline void launch_bsr3(cudaStream_t s, int nrows, const int32_t *rowptr, const int32_t *colidx,
+inline void launch_bsr3(cudaStream_t s, int sharers, int nrows, const int32_t *rowptr, const int32_t *colidx,
                         const MT *val, const ST *x, const ST *b, const ST *dinv, const ST *binv, ST *y,
                         const GmresState *st, int j, const double *xscale, const int *active = nullptr)
 {
-  if (nrows <= BSR3_WARPS)
+  if ((int64_t)nrows * sharers <= BSR3_WARPS)
     bsr3_spmv<MODE, PC, MT, ST><<<(int)((nrows * 32LL + 255) / 256), 256, 0, s>>>(nrows, rowptr, colidx, val, x, b, dinv, binv, y, st, j, xscale, active);
   else
     bsr3_spmv_rows<MODE, PC, MT, ST><<<(int)((nrows * 3LL + 255) / 256), 256, 0, s>>>(nrows, rowptr, colidx, val, x, b, dinv, binv, y, st, j, xscale, active);
@@ -674,11 +675,84 @@ gmres_mdot_each(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, co
   }
 }
 
+// The same sums, in the same order, for instances that share the chip (a batch):
+// there no SM is idle and what counts is the work, so a CTA of 256 threads takes
+// MDOT_SHARED vectors and reads w once for them.  Thread t does the part of threads
+// t, t + 256, .. of a CTA of NT.  With a CTA per vector 64 instances of 12,675
+// unknowns (up to 200 vectors) took 133 ms a step instead of 118.
+constexpr int MDOT_SHARED = 4;
+inline bool mdot_shared(int threads, int vectors, int sharers)
+{
+  return sharers > 1 && (int64_t)sharers * vectors * threads > 148 * 2048;
+}
+template <typename VT, int NT>
+__global__ void __launch_bounds__(ORTHO_THREADS)
+gmres_mdot_shared(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, const GmresState *__restrict__ st,
+                  GmresArrays ga)
+{
+  if (!st->active || st->it != j) return;
+  constexpr int E = Chunk<VT>::E, VEC = MDOT_SHARED, PARTS = NT / ORTHO_THREADS, W = ORTHO_THREADS / 32;
+  constexpr int UN = PARTS > 1 ? 2 : 1;      // parts whose loads are in flight together
+  static_assert(PARTS % UN == 0, "");
+  __shared__ double sh[VEC][NT / 32];
+  const int k0 = blockIdx.x * VEC;
+  const VT *w = V + (int64_t)(j + 1) * ldv;
+  const VT *v[VEC];
+#pragma unroll
+  for (int i = 0; i < VEC; i++) v[i] = V + (int64_t)min(k0 + i, j) * ldv;
+  double acc[PARTS][VEC] = {};
+  for (int64_t p0 = threadIdx.x; p0 < nchunk; p0 += NT) {
+#pragma unroll
+    for (int q0 = 0; q0 < PARTS; q0 += UN) {
+      double a[UN][VEC][E], b[UN][E];
+#pragma unroll
+      for (int q = 0; q < UN; q++) {
+        const int64_t p = p0 + (q0 + q) * ORTHO_THREADS;
+        if (p < nchunk) {
+          Chunk<VT>::load(w + E * p, b[q]);
+#pragma unroll
+          for (int i = 0; i < VEC; i++) Chunk<VT>::load(v[i] + E * p, a[q][i]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < UN; q++) {
+        if (p0 + (q0 + q) * ORTHO_THREADS < nchunk) {
+#pragma unroll
+          for (int i = 0; i < VEC; i++)
+#pragma unroll
+            for (int e = 0; e < E; e++) acc[q0 + q][i] = fma(a[q][i][e], b[q][e], acc[q0 + q][i]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < PARTS; q++)
+#pragma unroll
+    for (int i = 0; i < VEC; i++) {
+      double t = acc[q][i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (threadIdx.x % 32 == 0) sh[i][q * W + threadIdx.x / 32] = t;
+    }
+  __syncthreads();
+  const int k = k0 + threadIdx.x;
+  if (threadIdx.x < VEC && k <= j) {
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < NT / 32; q++) t += sh[threadIdx.x][q];
+    const double sigma = ga.sigma[k];
+    const double hkj = sigma * t;
+    ga.H[hidx(k, j, st->m)] = hkj;
+    ga.coef[k] = hkj * sigma;
+  }
+}
+
 // w -= sum_k h_k sigma_k V_k, then ||w||^2 partials.  A CTA covers CL * PER
-// 16-byte chunks; its threads are 256 / CL groups of CL: group g adds the k's
-// congruent to g modulo the number of groups, each thread for its PER chunks,
-// UN terms in flight, and the groups' sums are combined in a fixed order
-// through shared memory.  One more CTA applies the stored Givens rotations to
+// 16-byte chunks; its threads are 256 / CL sets of CL, and the k's fall into
+// 256 / CL * RES groups, the residues of k modulo their number, RES of them to a
+// set: a thread adds the terms of each of its groups for its PER chunks, UN * RES
+// terms in flight, and the groups' sums are combined in a fixed order through
+// shared memory.  One more CTA, the first, applies the stored Givens rotations to
 // column j meanwhile (a serial chain of j steps, none of which needs the norm);
 // the last CTA to arrive finishes the norm, forms the new rotation and runs the
 // convergence test (KSPGMRESUpdateHessenberg, KSPConvergedDefault).  The last step
@@ -690,12 +764,17 @@ gmres_mdot_each(int64_t nchunk, const VT *__restrict__ V, int64_t ldv, int j, co
 // groups, which fills the SMs and cuts the chain to j / 128 batches.
 // With the wide form for every size and the rotations after the norm: 6.5 us at 363
 // unknowns and 50 vectors, 15.5 at 10,092 and 300; now 5.0 and 7.5.
+//
+// The packed form (128 x 1, eight groups a thread) has an eighth of the narrow one's
+// CTAs and the same 16 groups and partial sums, so the same bits.
 constexpr int ROT_PER = 1024 / ORTHO_THREADS;      // columns per thread of the rotations (restart <= 1000)
 constexpr int MAXPY_FEW_SPAN = 16, MAXPY_WIDE_SPAN = 128;
 // The narrow form pays while its CTAs, three an SM, are resident at once (14,208 FP64
 // unknowns): a step of the hex8 cavity with 19,652 and 37,044 unknowns took 9.6 and
 // 13.6 ms with it and 8.8 and 11.0 with the wide one, quad4 with 30,603 25.8 and 23.2;
-// with 12,675 5.9 and 6.9 the other way.
+// with 12,675 5.9 and 6.9 the other way.  Instances that share the chip fill it
+// together: 64 of 12,675 unknowns 148 ms a step with the narrow form, 118 with the
+// packed one, 32 hex8 of 8,788 30.8 and 24.3.
 constexpr int MAXPY_WAVE = 3 * 148;
 constexpr int64_t MAXPY_FEW = (int64_t)MAXPY_FEW_SPAN * MAXPY_WAVE;
 inline int maxpy_tiles(int64_t nchunk, bool few)
@@ -703,8 +782,9 @@ inline int maxpy_tiles(int64_t nchunk, bool few)
   const int span = few ? MAXPY_FEW_SPAN : MAXPY_WIDE_SPAN;
   return (int)((nchunk + span - 1) / span);
 }
-template <typename VT, int CL, int PER, int UN>
-__global__ void __launch_bounds__(ORTHO_THREADS, PER > 1 ? 5 : 3)
+inline bool maxpy_narrow(int64_t nchunk, int sharers) { return (int64_t)maxpy_tiles(nchunk, true) * sharers <= MAXPY_WAVE; }
+template <typename VT, int CL, int PER, int UN, int RES>
+__global__ void __launch_bounds__(ORTHO_THREADS, PER > 1 ? 5 : RES > 1 ? 2 : 3)
 gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresState *st, GmresArrays ga,
                  GmresState *snap)
 {
@@ -712,8 +792,9 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
     if (snap && blockIdx.x == 0 && threadIdx.x == 0) *snap = *st;
     return;
   }
-  constexpr int E = Chunk<VT>::E, SPAN = CL * PER, GROUPS = ORTHO_THREADS / CL;
-  static_assert(SPAN <= ORTHO_THREADS, "");
+  constexpr int E = Chunk<VT>::E, SPAN = CL * PER, GROUPS = ORTHO_THREADS / CL * RES;
+  constexpr int TILE = RES > 1 ? MAXPY_FEW_SPAN : SPAN;    // chunks of a partial sum
+  static_assert(SPAN <= ORTHO_THREADS && (RES == 1 || (GROUPS == ORTHO_THREADS / MAXPY_FEW_SPAN && TILE == 16)), "");
   __shared__ double sh[ORTHO_THREADS / 32];
   __shared__ union {
     double qs[GROUPS][E][SPAN];
@@ -723,8 +804,7 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
     } rot;                         // the CTA of the rotations
   } u;
   const int m = st->m;
-  const int tiles = (int)gridDim.x - 1;
-  if ((int)blockIdx.x == tiles) {
+  if (blockIdx.x == 0) {
     // a_0 = h_0, a_{q+1} = c_q h_{q+1} - s_q a_q is the chain; the products
     // before it and the rotated entries c_q a_q + s_q h_{q+1} after it take all threads
     double2 *st2 = u.rot.step;
@@ -771,14 +851,14 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
     const double *__restrict__ hk = ga.coef;
     VT *w = V + (int64_t)(j + 1) * ldv;
     const int lp = threadIdx.x % CL, g = threadIdx.x / CL;
-    const int64_t c0 = (int64_t)blockIdx.x * SPAN;
+    const int64_t c0 = (int64_t)(blockIdx.x - 1) * SPAN;
     // the chunk of w this thread finishes, loaded early; nchunk is a multiple
     // of 16 (ldv is one of 32 entries), the spans may reach past it
     const int64_t pfin = c0 + threadIdx.x;
     const bool fin = threadIdx.x < SPAN && pfin < nchunk;
     double wfin[E];
     if (fin) Chunk<VT>::load(w + E * pfin, wfin);
-    double acc[PER][E] = {};
+    double acc[RES][PER][E] = {};
     const VT *bp[PER];
     bool in[PER];
 #pragma unroll
@@ -788,32 +868,38 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
       bp[i] = V + E * (in[i] ? p : c0);
     }
     if (in[0]) {
-      for (int k = g; k <= j; k += GROUPS * UN) {
-        double v[UN][PER][E], c[UN];
+      for (int k = g * RES; k <= j; k += GROUPS * UN) {
+        double v[UN][RES][PER][E], c[UN][RES];
 #pragma unroll
-        for (int t = 0; t < UN; t++) {
-          const int kt = k + t * GROUPS;
-          if (kt <= j) {
-            c[t] = __ldg(hk + kt);
+        for (int t = 0; t < UN; t++)
 #pragma unroll
-            for (int i = 0; i < PER; i++) Chunk<VT>::load(bp[i] + (int64_t)kt * ldv, v[t][i]);
+          for (int r = 0; r < RES; r++) {
+            const int kt = k + t * GROUPS + r;
+            if (kt <= j) {
+              c[t][r] = __ldg(hk + kt);
+#pragma unroll
+              for (int i = 0; i < PER; i++) Chunk<VT>::load(bp[i] + (int64_t)kt * ldv, v[t][r][i]);
+            }
           }
-        }
 #pragma unroll
-        for (int t = 0; t < UN; t++) {
-          if (k + t * GROUPS <= j) {
+        for (int t = 0; t < UN; t++)
 #pragma unroll
-            for (int i = 0; i < PER; i++)
+          for (int r = 0; r < RES; r++) {
+            if (k + t * GROUPS + r <= j) {
 #pragma unroll
-              for (int e = 0; e < E; e++) acc[i][e] = fma(c[t], v[t][i][e], acc[i][e]);
+              for (int i = 0; i < PER; i++)
+#pragma unroll
+                for (int e = 0; e < E; e++) acc[r][i][e] = fma(c[t][r], v[t][r][i][e], acc[r][i][e]);
+            }
           }
-        }
       }
     }
 #pragma unroll
-    for (int i = 0; i < PER; i++)
+    for (int r = 0; r < RES; r++)
 #pragma unroll
-      for (int e = 0; e < E; e++) u.qs[g][e][lp + i * CL] = acc[i][e];
+      for (int i = 0; i < PER; i++)
+#pragma unroll
+        for (int e = 0; e < E; e++) u.qs[g * RES + r][e][lp + i * CL] = acc[r][i][e];
     __syncthreads();
     double s = 0.0;
     if (fin) {
@@ -837,13 +923,20 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
         s = fma(v, v, s);
       }
     }
-    s = block_sum<ORTHO_THREADS>(s, sh);
-    if (threadIdx.x == 0) ga.partial[blockIdx.x] = s;
+    if constexpr (RES > 1) {
+      // half a warp each: the order of block_sum over 16 threads
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (fin && threadIdx.x % TILE == 0) ga.partial[pfin / TILE] = s;
+    } else {
+      s = block_sum<ORTHO_THREADS>(s, sh);
+      if (threadIdx.x == 0) ga.partial[blockIdx.x - 1] = s;
+    }
   }
   if (last_block(&st->counter, gridDim.x)) {
     double a = 0.0, g0 = 0.0;
     if (threadIdx.x == 0) { a = __ldcg(ga.H + hidx(j, j, m)); g0 = __ldcg(ga.grs + j); }
-    const double t = sum_partials(ga.partial, tiles, sh);
+    const double t = sum_partials(ga.partial, (unsigned int)((nchunk + TILE - 1) / TILE), sh);
     if (threadIdx.x == 0) {
       const int it = j;
       const double tt = sqrt(t);
