@@ -119,6 +119,7 @@ struct cfdgpu_handle {
   IluPattern ilu;
   int32_t *frow = nullptr, *fcol = nullptr, *fdiag = nullptr, *faslot = nullptr;
   uint32_t *fumap = nullptr;
+  uint64_t *fumap64 = nullptr;
   double *frowbuf = nullptr;       // factorisation rows that do not fit into shared memory
   int32_t *florder = nullptr, *fperm = nullptr;
   TrsvView plan_l{}, plan_u{};     // schedules of the lower and upper solve: groups of rows,
@@ -460,7 +461,7 @@ static double ilu_factor_bytes(cfdgpu_handle *h)
   // read A and the update map once, write the factors and the inverted diagonals once
   const double bb = (double)h->ndof * h->ndof * 8.0;
   return (double)h->topo.nnzb() * bb + (double)h->ilu.nnzb() * bb + (double)h->nNode * bb +
-         4.0 * (double)h->ilu.umap.size() + 8.0 * (double)h->ilu.uoff.size();
+         4.0 * (double)h->ilu.umap.size() + 8.0 * (double)(h->ilu.umap64.size() + h->ilu.uoff.size());
 }
 
 static double trsv_bytes(cfdgpu_handle *h)
@@ -502,10 +503,14 @@ static int ilu_factor_t(cfdgpu_handle *h, const T *a, T *fval, T *fdinv)
 {
   const int pi = prof_begin(h, CFDGPU_KIND_ILU, ilu_factor_bytes(h) * (sizeof(T) / 8.0));
   const FactorLaunch f = factor_launch(h);
-  const auto kernel = f.wide ? ilu_factor<NB, T, T, true> : ilu_factor<NB, T, T, false>;
-  kernel<<<f.grid, 32 * f.warps, f.smem, h->stream>>>(
-      h->nNode, h->ilu.maxrow, h->rowptr, h->faslot, a, h->frow, h->fcol, h->fdiag, h->fuoff, h->fumap, h->florder,
-      h->fperm, fval, fdinv, h->iflags, h->tctl, h->frowbuf);
+  auto run = [&](auto kernel, auto *umap) {
+    kernel<<<f.grid, 32 * f.warps, f.smem, h->stream>>>(h->nNode, h->ilu.maxrow, h->rowptr, h->faslot, a, h->frow, h->fcol,
+                                                        h->fdiag, h->fuoff, umap, h->florder, h->fperm, fval, fdinv,
+                                                        h->iflags, h->tctl, h->frowbuf);
+  };
+  if (h->fumap64) run(ilu_factor<NB, T, T, true, uint64_t>, h->fumap64);
+  else if (f.wide) run(ilu_factor<NB, T, T, true, uint32_t>, h->fumap);
+  else run(ilu_factor<NB, T, T, false, uint32_t>, h->fumap);
   prof_end(h, pi);
   LAUNCHED(h);
   return check_launch(h, "ilu_factor");
@@ -531,8 +536,9 @@ static int ilu_limits(cfdgpu_handle *h)
   auto most = [](auto kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  CK(most(ilu_factor<NB, T, T, true>, FACTOR_SMEM));
-  CK(most(ilu_factor<NB, T, T, false>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, true, uint64_t>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, true, uint32_t>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, false, uint32_t>, FACTOR_SMEM));
   CK(most(ilu_trsv<NB, false, T>, TRSV_SMEM));
   CK(most(ilu_trsv<NB, true, T>, TRSV_SMEM));
   return 0;
@@ -1408,7 +1414,11 @@ int cfdgpu_create(const cfdgpu_mesh *mesh, const cfdgpu_control *ctrl, const cfd
     if ((rc = upload(h, &h->fdiag, f.diag.data(), f.diag.size()))) return rc;
     if ((rc = upload(h, &h->faslot, f.aslot.data(), f.aslot.size()))) return rc;
     if ((rc = upload(h, &h->fuoff, f.uoff.data(), f.uoff.size()))) return rc;
-    if ((rc = upload(h, &h->fumap, f.umap.data(), f.umap.size()))) return rc;
+    if (!f.umap64.empty()) {
+      if ((rc = upload(h, &h->fumap64, f.umap64.data(), f.umap64.size()))) return rc;
+    } else if ((rc = upload(h, &h->fumap, f.umap.data(), f.umap.size()))) {
+      return rc;
+    }
     if ((rc = upload(h, &h->florder, f.lorder.data(), f.lorder.size()))) return rc;
     if ((rc = ilu_limits(h))) return rc;
     if ((rc = upload_trsv(h, false, h->plan_l, h->chain_l)) || (rc = upload_trsv(h, true, h->plan_u, h->chain_u))) return rc;

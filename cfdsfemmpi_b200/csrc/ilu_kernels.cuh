@@ -169,7 +169,7 @@ __device__ __forceinline__ double invert_block(const double *A, int lane, bool &
 // p < i of the row in increasing column order, L_ip = W_p U_pp^-1 and
 // W_j -= L_ip U_pj for the blocks j > p of row p that lie in row i's pattern
 // (list umap: the block's number in row p after the diagonal, and its place in
-// row i); then U_ii^-1.  AT is the type of the assembled matrix, FT of the
+// row i: the halves of an ENT); then U_ii^-1.  AT is the type of the assembled matrix, FT of the
 // factors; W is FP64 and lives in shared memory (in `scratch` when a row does
 // not fit).
 //
@@ -190,17 +190,19 @@ __device__ __forceinline__ double invert_block(const double *A, int lane, bool &
 // registers: complete LU of the 64 x 64 cavity 24.1 -> 18.9 ms.  On shorter rows
 // more rounds only cost registers (four on the O-grid: 4.5 -> 4.8 ms).
 constexpr int factor_wide(int nb) { return 4 * (32 / nb) * 2; }
-template <int NB, typename AT, typename FT, bool WIDE>
+template <int NB, typename AT, typename FT, bool WIDE, typename ENT>
 __global__ void __launch_bounds__(ILU_THREADS, WIDE ? 1 : 2)
 ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *__restrict__ aslot,
            const AT *__restrict__ aval, const int32_t *__restrict__ fptr, const int32_t *__restrict__ fcol,
-           const int32_t *__restrict__ fdiag, const int64_t *__restrict__ uoff, const uint32_t *__restrict__ umap,
+           const int32_t *__restrict__ fdiag, const int64_t *__restrict__ uoff, const ENT *__restrict__ umap,
            const int32_t *__restrict__ order, const int32_t *__restrict__ perm, FT *fval, FT *fdinv,
            unsigned int *flags, TriCtl *ctl, double *scratch)
 {
   constexpr int BB = NB * NB;
   constexpr int PER = 32 / NB;        // blocks updated at once: lane = (block, row)
   constexpr int UNR = WIDE ? (NB == 3 ? 7 : 4) : 2;
+  constexpr int HALF = 4 * sizeof(ENT);      // bits of a block's place in the row
+  constexpr ENT NONE = ~ENT(0), PLACE = NONE >> HALF;
   extern __shared__ __align__(16) double wsm[];
   __shared__ double Lsh[ILU_WARPS][BB];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -243,11 +245,11 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
       const int64_t o0 = __shfl_sync(0xffffffffu, ul, b), o1 = __shfl_sync(0xffffffffu, un, b);
       const int u0 = fdiag[p] + 1;
       // this lane's first blocks: entries of the list do not depend on the pivot's values
-      uint32_t ent[UNR];
+      ENT ent[UNR];
 #pragma unroll
       for (int k = 0; k < UNR; k++) {
         const int64_t o = o0 + k * PER + ob;
-        ent[k] = ob < PER && o < o1 ? umap[o] : 0xffffffffu;
+        ent[k] = ob < PER && o < o1 ? umap[o] : NONE;
       }
       if (!((done >> b) & 1u)) {
         wait_flag(flags + p, target, ctl);
@@ -260,9 +262,9 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
 #pragma unroll
       for (int k = 0; k < NB; k++) dcol[k] = (double)__ldcg(fdinv + (int64_t)p * BB + k * NB + ec);
       auto fetch = [&](int k) {
-        if (ent[k] != 0xffffffffu) {
+        if (ent[k] != NONE) {
 #pragma unroll
-          for (int c = 0; c < NB; c++) ld_row<NB>(fval + (int64_t)(u0 + (int)(ent[k] >> 16)) * BB + c * NB, ub[k][c]);
+          for (int c = 0; c < NB; c++) ld_row<NB>(fval + (int64_t)(u0 + (int)(ent[k] >> HALF)) * BB + c * NB, ub[k][c]);
         }
       };
 #pragma unroll
@@ -281,8 +283,8 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
       for (int64_t o = o0; o < o1; o += PER * UNR) {
 #pragma unroll
         for (int k = 0; k < UNR; k++) {
-          if (ent[k] != 0xffffffffu) {
-            double *const t = W + (ent[k] & 0xffffu) * BB + orow * NB;
+          if (ent[k] != NONE) {
+            double *const t = W + (int)(ent[k] & PLACE) * BB + orow * NB;
 #pragma unroll
             for (int c = 0; c < NB; c++) {
               double s = 0.0;
@@ -296,7 +298,7 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
 #pragma unroll
           for (int k = 0; k < UNR; k++) {
             const int64_t x = o + PER * (UNR + k) + ob;
-            ent[k] = ob < PER && x < o1 ? umap[x] : 0xffffffffu;
+            ent[k] = ob < PER && x < o1 ? umap[x] : NONE;
           }
 #pragma unroll
           for (int k = 0; k < UNR; k++) fetch(k);

@@ -2,6 +2,7 @@
 #include "setup.h"
 
 #include <algorithm>
+#include <type_traits>
 #include <climits>
 #include <cstdint>
 #include <numeric>
@@ -333,25 +334,29 @@ std::string build_ilu_pattern(const Topology &t, int levels, int nblocks, IluPat
   // update lists: the upper blocks of every pivot row that row i's pattern holds
   {
     for (int i = 0; i < n; i++) f.maxrow = std::max(f.maxrow, f.rowptr[i + 1] - f.rowptr[i]);
-    if (f.maxrow > 65535) return "ILU row of more than 65535 blocks";
     f.uoff.resize(f.colidx.size() + 1);
     int64_t most = 0;
     for (int i = 0; i < n; i++)
       for (int q = f.rowptr[i]; q < f.diag[i]; q++) most += f.rowptr[f.colidx[q] + 1] - f.diag[f.colidx[q]] - 1;
-    f.umap.reserve((size_t)most);
-    std::vector<int32_t> pos(n, -1);
-    for (int i = 0; i < n; i++) {
-      for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = k - f.rowptr[i];
-      for (int q = f.rowptr[i]; q < f.rowptr[i + 1]; q++) {
-        f.uoff[q] = (int64_t)f.umap.size();
-        if (q >= f.diag[i]) continue;
-        const int p = f.colidx[q], u0 = f.diag[p] + 1;
-        for (int u = u0; u < f.rowptr[p + 1]; u++)
-          if (pos[f.colidx[u]] >= 0) f.umap.push_back((uint32_t)(u - u0) << 16 | (uint32_t)pos[f.colidx[u]]);
+    auto list = [&](auto &map) {
+      using E = typename std::decay_t<decltype(map)>::value_type;
+      map.reserve((size_t)most);
+      std::vector<int32_t> pos(n, -1);
+      for (int i = 0; i < n; i++) {
+        for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = k - f.rowptr[i];
+        for (int q = f.rowptr[i]; q < f.rowptr[i + 1]; q++) {
+          f.uoff[q] = (int64_t)map.size();
+          if (q >= f.diag[i]) continue;
+          const int p = f.colidx[q], u0 = f.diag[p] + 1;
+          for (int u = u0; u < f.rowptr[p + 1]; u++)
+            if (pos[f.colidx[u]] >= 0) map.push_back((E)(u - u0) << 4 * sizeof(E) | (E)pos[f.colidx[u]]);
+        }
+        for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = -1;
       }
-      for (int k = f.rowptr[i]; k < f.rowptr[i + 1]; k++) pos[f.colidx[k]] = -1;
-    }
-    f.uoff[f.colidx.size()] = (int64_t)f.umap.size();
+      f.uoff[f.colidx.size()] = (int64_t)map.size();
+    };
+    if (f.maxrow > 65535) list(f.umap64);
+    else list(f.umap);
   }
   // blocks of A inside the factor pattern (A's block (v, c) lands in factor
   // row IP(v) at column IP(c))

@@ -69,9 +69,10 @@ struct IluPattern {
   // updates of the numeric factorisation: for a strictly lower block q = (i, p),
   // umap[uoff[q]..uoff[q+1]) lists the blocks of row p right of its diagonal that
   // lie in row i's pattern: their number after the diagonal << 16 | their place
-  // in row i
+  // in row i; where a row has more than 65,535 blocks, umap64 instead, << 32
   std::vector<int64_t> uoff;     // nnzb + 1
   std::vector<uint32_t> umap;
+  std::vector<uint64_t> umap64;
   int maxrow = 0;                // blocks of the longest row
   // rows sorted by level of the lower DAG (factorisation and lower solve:
   // level(i) = 1 + max level of the strictly lower blocks' columns) and of
