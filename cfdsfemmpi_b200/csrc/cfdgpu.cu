@@ -41,6 +41,21 @@ struct DevBuf {
 
 }  // namespace
 
+// Shared memory for one warp's row of the factorisation, warps per CTA and
+// CTAs: as many warps as the rows leave room for (8 at most, two CTAs per SM),
+// and no more than twice the widest dependency level holds (at least 256), since
+// warps beyond what the levels can feed only add polling traffic.  Where the longest
+// row does not fit, eight warps' shares hold the shorter rows, and the longer ones
+// have places in memory: each its own if they are few, else one per warp.
+constexpr size_t FACTOR_SMEM = 220 * 1024;    // for rows, of the 227 KB that a CTA may have
+struct FactorLaunch {
+  int warps, grid;
+  size_t smem;
+  int rowcap;          // blocks of a row in shared memory
+  int64_t places;      // rows in memory
+  bool by_row, wide;
+};
+
 struct cfdgpu_handle {
   std::string err;
   int ndim = 0, npe = 0, ndof = 0, nNode = 0, nElem = 0, et = 0;
@@ -120,7 +135,9 @@ struct cfdgpu_handle {
   int32_t *frow = nullptr, *fcol = nullptr, *fdiag = nullptr, *faslot = nullptr;
   uint32_t *fumap = nullptr;
   uint64_t *fumap64 = nullptr;
+  FactorLaunch flaunch{};
   double *frowbuf = nullptr;       // factorisation rows that do not fit into shared memory
+  int32_t *frowplace = nullptr;    // their places in it by row; NULL: by warp
   int32_t *florder = nullptr, *fperm = nullptr;
   TrsvView plan_l{}, plan_u{};     // schedules of the lower and upper solve: groups of rows,
   ChainView chain_l{}, chain_u{};  // or chains of rows (TrsvPlan::chains)
@@ -472,28 +489,23 @@ static double trsv_bytes(cfdgpu_handle *h)
   return (double)h->ilu.nnzb() * (bb + 4.0) + (double)h->nNode * bb + 4.0 * V;
 }
 
-// Shared memory for one warp's row of the factorisation, warps per CTA and
-// CTAs: as many warps as the rows leave room for (8 at most, two CTAs per SM),
-// and no more than twice the widest dependency level holds (at least 256), since
-// warps beyond what the levels can feed only add polling traffic.
-constexpr size_t FACTOR_SMEM = 220 * 1024;    // for rows, of the 227 KB that a CTA may have
-struct FactorLaunch {
-  int warps, grid;
-  size_t smem;
-  bool in_smem, wide;
-};
 static FactorLaunch factor_launch(cfdgpu_handle *h)
 {
   constexpr size_t PER_SM = FACTOR_SMEM;
-  const size_t row = (size_t)h->ilu.maxrow * h->ndof * h->ndof * sizeof(double);
+  const size_t block = (size_t)h->ndof * h->ndof * sizeof(double), row = h->ilu.maxrow * block;
   FactorLaunch f;
-  f.in_smem = row <= PER_SM;
-  f.warps = f.in_smem ? (int)std::min<size_t>(ILU_WARPS, PER_SM / row) : ILU_WARPS;
-  f.smem = f.in_smem ? f.warps * row : 0;
+  const bool fits = row <= PER_SM;
+  f.warps = fits ? (int)std::min<size_t>(ILU_WARPS, PER_SM / row) : ILU_WARPS;
+  f.rowcap = fits ? h->ilu.maxrow : (int)(PER_SM / ILU_WARPS / block);
+  f.smem = f.warps * f.rowcap * block;
   f.wide = h->ilu.maxrow > factor_wide(h->ndof);
   const int per_sm = !f.wide && f.smem <= PER_SM / 2 ? 2 : 1;
   const int64_t want = std::min<int64_t>(h->nNode, std::max<int64_t>(256, 2 * (int64_t)h->ilu.maxw_l));
   f.grid = (int)std::max<int64_t>(1, std::min<int64_t>((want + f.warps - 1) / f.warps, 148 * per_sm));
+  f.places = 0;
+  for (int i = 0; i < h->nNode && !fits; i++) f.places += h->ilu.rowptr[i + 1] - h->ilu.rowptr[i] > f.rowcap;
+  f.by_row = f.places <= (int64_t)f.grid * f.warps;
+  f.places = std::min<int64_t>(f.places, (int64_t)f.grid * f.warps);
   return f;
 }
 
@@ -502,15 +514,16 @@ template <int NB, typename T>
 static int ilu_factor_t(cfdgpu_handle *h, const T *a, T *fval, T *fdinv)
 {
   const int pi = prof_begin(h, CFDGPU_KIND_ILU, ilu_factor_bytes(h) * (sizeof(T) / 8.0));
-  const FactorLaunch f = factor_launch(h);
+  const FactorLaunch &f = h->flaunch;
   auto run = [&](auto kernel, auto *umap) {
-    kernel<<<f.grid, 32 * f.warps, f.smem, h->stream>>>(h->nNode, h->ilu.maxrow, h->rowptr, h->faslot, a, h->frow, h->fcol,
+    kernel<<<f.grid, 32 * f.warps, f.smem, h->stream>>>(h->nNode, f.rowcap, h->rowptr, h->faslot, a, h->frow, h->fcol,
                                                         h->fdiag, h->fuoff, umap, h->florder, h->fperm, fval, fdinv,
-                                                        h->iflags, h->tctl, h->frowbuf);
+                                                        h->iflags, h->tctl, h->frowbuf, h->frowplace, h->ilu.maxrow);
   };
-  if (h->fumap64) run(ilu_factor<NB, T, T, true, uint64_t>, h->fumap64);
-  else if (f.wide) run(ilu_factor<NB, T, T, true, uint32_t>, h->fumap);
-  else run(ilu_factor<NB, T, T, false, uint32_t>, h->fumap);
+  if (h->fumap64) run(ilu_factor<NB, T, T, true, true, uint64_t>, h->fumap64);
+  else if (f.places) run(ilu_factor<NB, T, T, true, true, uint32_t>, h->fumap);
+  else if (f.wide) run(ilu_factor<NB, T, T, true, false, uint32_t>, h->fumap);
+  else run(ilu_factor<NB, T, T, false, false, uint32_t>, h->fumap);
   prof_end(h, pi);
   LAUNCHED(h);
   return check_launch(h, "ilu_factor");
@@ -536,9 +549,10 @@ static int ilu_limits(cfdgpu_handle *h)
   auto most = [](auto kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   };
-  CK(most(ilu_factor<NB, T, T, true, uint64_t>, FACTOR_SMEM));
-  CK(most(ilu_factor<NB, T, T, true, uint32_t>, FACTOR_SMEM));
-  CK(most(ilu_factor<NB, T, T, false, uint32_t>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, true, true, uint64_t>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, true, true, uint32_t>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, true, false, uint32_t>, FACTOR_SMEM));
+  CK(most(ilu_factor<NB, T, T, false, false, uint32_t>, FACTOR_SMEM));
   CK(most(ilu_trsv<NB, false, T>, TRSV_SMEM));
   CK(most(ilu_trsv<NB, true, T>, TRSV_SMEM));
   return 0;
@@ -1435,8 +1449,15 @@ int cfdgpu_create(const cfdgpu_mesh *mesh, const cfdgpu_control *ctrl, const cfd
       CK(cudaMemset(h->fdinv, 0, sizeof(double) * h->nNode * bb));
     }
     {
-      const FactorLaunch fl = factor_launch(h);
-      if (!fl.in_smem && (rc = dalloc(h, &h->frowbuf, (size_t)fl.grid * fl.warps * f.maxrow * bb))) return rc;
+      const FactorLaunch &fl = h->flaunch = factor_launch(h);
+      if (fl.places && (rc = dalloc(h, &h->frowbuf, (size_t)fl.places * f.maxrow * bb))) return rc;
+      if (fl.places && fl.by_row) {
+        std::vector<int32_t> place(h->nNode, -1);
+        int32_t k = 0;
+        for (int i = 0; i < h->nNode; i++)
+          if (f.rowptr[i + 1] - f.rowptr[i] > fl.rowcap) place[i] = k++;
+        if ((rc = upload(h, &h->frowplace, place.data(), place.size()))) return rc;
+      }
     }
     if ((rc = dalloc(h, &h->iflags, (size_t)h->nNode))) return rc;
     CK(cudaMemset(h->iflags, 0, sizeof(unsigned int) * h->nNode));

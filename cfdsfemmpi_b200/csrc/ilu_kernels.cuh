@@ -169,9 +169,9 @@ __device__ __forceinline__ double invert_block(const double *A, int lane, bool &
 // p < i of the row in increasing column order, L_ip = W_p U_pp^-1 and
 // W_j -= L_ip U_pj for the blocks j > p of row p that lie in row i's pattern
 // (list umap: the block's number in row p after the diagonal, and its place in
-// row i: the halves of an ENT); then U_ii^-1.  AT is the type of the assembled matrix, FT of the
-// factors; W is FP64 and lives in shared memory (in `scratch` when a row does
-// not fit).
+// row i: the halves of an ENT); then U_ii^-1.  AT is the type of the assembled
+// matrix, FT of the factors; W is FP64 and lives in shared memory (with PLACES, rows
+// of more than rowcap blocks in `scratch`).
 //
 // What bounds it: the dependency chain, per level the last pivot's hop.  With W
 // in global memory, one fence per pivot and the inverse by one lane the kernel
@@ -180,23 +180,27 @@ __device__ __forceinline__ double invert_block(const double *A, int lane, bool &
 // the complete LU of the 64 x 64 cavity (4,224 levels).  Now a pivot's inverse and
 // the blocks of its row are requested together once its flag is seen (pivots long
 // done are found by one poll of all flags), and the row's blocks that others need
-// are written and published before the rest: 3.5, 1.5, 0.25, 4.5 and 18.9 ms (FP32
+// are written and published before the rest: 2.9, 1.2, 0.25, 4.5 and 17.1 ms (FP32
 // values are rounded where they were stored before, so the factors keep their bits).
+// An instance whose rows all fit has no PLACES, and its accesses to W are known to be
+// to shared memory: with a pointer to either it took 3.5, 1.5, 0.26, 4.5 and 18.8.
 //
 // UNR rounds of 32 / NB blocks are fetched at once.  Where a pivot's list takes more
 // than two fetches of two rounds (rows of over factor_wide(NB) blocks: complete LU,
 // high levels) the last pivot's fetches are on the chain one after another, and the
 // WIDE form fetches seven rounds (four of 4x4 blocks) with one CTA per SM for the
-// registers: complete LU of the 64 x 64 cavity 24.1 -> 18.9 ms.  On shorter rows
+// registers: complete LU of the 64 x 64 cavity 24.1 -> 18.9 ms (before the above).
+// Seven rounds are 70 blocks of 3x3; a pivot's list has 84 on average there and the
+// rest of it comes in a second fetch.  On shorter rows
 // more rounds only cost registers (four on the O-grid: 4.5 -> 4.8 ms).
 constexpr int factor_wide(int nb) { return 4 * (32 / nb) * 2; }
-template <int NB, typename AT, typename FT, bool WIDE, typename ENT>
+template <int NB, typename AT, typename FT, bool WIDE, bool PLACES, typename ENT>
 __global__ void __launch_bounds__(ILU_THREADS, WIDE ? 1 : 2)
 ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *__restrict__ aslot,
            const AT *__restrict__ aval, const int32_t *__restrict__ fptr, const int32_t *__restrict__ fcol,
            const int32_t *__restrict__ fdiag, const int64_t *__restrict__ uoff, const ENT *__restrict__ umap,
            const int32_t *__restrict__ order, const int32_t *__restrict__ perm, FT *fval, FT *fdinv,
-           unsigned int *flags, TriCtl *ctl, double *scratch)
+           unsigned int *flags, TriCtl *ctl, double *scratch, const int32_t *__restrict__ place, int maxrow)
 {
   constexpr int BB = NB * NB;
   constexpr int PER = 32 / NB;        // blocks updated at once: lane = (block, row)
@@ -206,8 +210,6 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
   extern __shared__ __align__(16) double wsm[];
   __shared__ double Lsh[ILU_WARPS][BB];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  double *const W = scratch ? scratch + (int64_t)(blockIdx.x * (blockDim.x / 32) + w) * rowcap * BB
-                            : wsm + (int64_t)w * rowcap * BB;
   const unsigned int epoch = *(volatile unsigned int *)&ctl->epoch;
   const unsigned int target = epoch + 1u;
   const int e = lane % BB, er = e / NB, ec = e % NB;
@@ -217,6 +219,10 @@ ilu_factor(int n, int rowcap, const int32_t *__restrict__ arow, const int32_t *_
     if (tk >= n) break;
     const int i = order[tk];
     const int f0 = fptr[i], f1 = fptr[i + 1], fd = fdiag[i];
+    double *W = wsm + (int64_t)w * rowcap * BB;
+    if constexpr (PLACES) {
+      if (f1 - f0 > rowcap) W = scratch + (int64_t)(place ? place[i] : blockIdx.x * (blockDim.x / 32) + w) * maxrow * BB;
+    }
     for (int x = lane; x < (f1 - f0) * BB; x += 32) W[x] = 0.0;
     __syncwarp();
     {

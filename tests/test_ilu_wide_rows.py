@@ -63,3 +63,24 @@ def test_factors_of_wide_rows_multiply_to_the_matrix(ndim, length):
 @pytest.mark.parametrize("ndim,length", CASES)
 def test_solves_with_wide_rows_invert_the_factors(ndim, length):
     check_solves("wide", lambda: _strip(ndim, length), -1, 2)
+
+
+@pytest.mark.gpu
+def test_a_few_wide_rows_take_little_memory():
+    """What the complete factorisation takes beyond ILU(0) of the same strip: for a block of the factors 128 bytes for its
+    value, 12 for its indices, 72 for its list of at most nine updates and 12 for its part of the solves' records; nine
+    places for rows of 65,700 blocks of 128 bytes; and 2 MB for the rounding of each of some 60 allocations.  (A place
+    for each of 256 warps would be 2.2 GB.)"""
+    torch = pytest.importorskip("torch")
+    from cfdsfemmpi_b200 import Handle
+    mesh = _strip(3, 14600)
+    torch.zeros(1, device="cuda")
+    used, nnz = [], []
+    for levels in (0, -1):
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        h = Handle(mesh, meshgen.control_for(5, 0.1, 0.01), ksp="preonly", pc="bjacobi", ilu_levels=levels, bjacobi_blocks=2)
+        used.append(before - torch.cuda.mem_get_info()[0])
+        nnz.append(h.ilu_factors(values=False)["colidx"].size)
+        h.close()
+    assert used[1] - used[0] <= 224 * (nnz[1] - nnz[0]) + 9 * 65700 * 128 + 60 * 2 ** 21
