@@ -571,9 +571,9 @@ static int upload_trsv(cfdgpu_handle *h, bool upper, TrsvView &V, ChainView &C)
   build_trsv_plan(h->ilu, h->ndof, upper, p, true);
   if (p.chains) {
     const std::vector<int32_t> &ch = upper ? h->ilu.uchain : h->ilu.lchain;
-    const std::vector<int32_t> &ord = upper ? h->ilu.uchain_order : h->ilu.lchain_order;
+    int levels, rc;
+    const std::vector<int32_t> ord = chain_order(h->ilu, upper, levels);
     int32_t *chains, *order;
-    int rc;
     if ((rc = upload(h, &chains, ch.data(), ch.size())) || (rc = upload(h, &order, ord.data(), ord.size()))) return rc;
     C.chains = chains; C.order = order;
     C.nchains = (int)ord.size();
@@ -1856,15 +1856,15 @@ int cfdgpu_ilu_pattern_build(const cfdgpu_mesh *mesh, int levels, int nblocks, c
   if (!msg.empty()) return CFDGPU_EINVAL;
   info->nNode = mesh->nNode;
   info->nnzb = f.nnzb();
-  info->nchains_l = (int)f.lchain_order.size();
-  info->nchains_u = (int)f.uchain_order.size();
+  const std::vector<int32_t> lorder_c = chain_order(f, false, info->chain_levels_l);
+  const std::vector<int32_t> uorder_c = chain_order(f, true, info->chain_levels_u);
+  info->nchains_l = (int)lorder_c.size();
+  info->nchains_u = (int)uorder_c.size();
   info->nlev_l = f.nlev_l;
   info->nlev_u = f.nlev_u;
-  info->chain_levels_l = f.lchain_levels;
-  info->chain_levels_u = f.uchain_levels;
   auto cp = [](int32_t *dst, const std::vector<int32_t> &v) { if (dst && !v.empty()) memcpy(dst, v.data(), v.size() * 4); };
   cp(rowptr, f.rowptr); cp(colidx, f.colidx); cp(lorder, f.lorder); cp(uorder, f.uorder);
-  cp(lchain, f.lchain); cp(uchain, f.uchain); cp(lchain_order, f.lchain_order); cp(uchain_order, f.uchain_order);
+  cp(lchain, f.lchain); cp(uchain, f.uchain); cp(lchain_order, lorder_c); cp(uchain_order, uorder_c);
   if (perm) {
     if (f.perm.empty())
       for (int i = 0; i < mesh->nNode; i++) perm[i] = i;

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <type_traits>
+#include <utility>
 #include <climits>
 #include <cstdint>
 #include <numeric>
@@ -272,64 +273,24 @@ std::string build_ilu_pattern(const Topology &t, int levels, int nblocks, IluPat
       lev[i] = d;
     }
     f.nlev_l = order_by(f.lorder, f.maxw_l);
+    f.llev = lev;
     for (int i = n - 1; i >= 0; i--) {
       int d = 0;
       for (int q = f.diag[i] + 1; q < f.rowptr[i + 1]; q++) d = std::max(d, lev[f.colidx[q]] + 1);
       lev[i] = d;
     }
     f.nlev_u = order_by(f.uorder, f.maxw_u);
+    f.ulev = std::move(lev);
   }
-  // chains of the lower (ascending) and upper (descending) solves and their
-  // DAG levels
-  {
-    auto chains = [&](bool upper, std::vector<int32_t> &ch, std::vector<int32_t> &order, int &nlev, int &maxw) {
-      ch.clear();
-      std::vector<int32_t> chain_of(n);
-      if (!upper) {
-        int start = 0;
-        for (int i = 1; i <= n; i++) {
-          const bool cont = i < n && i - start < ILU_CHAIN_MAX && f.diag[i] > f.rowptr[i] &&
-                            f.colidx[f.diag[i] - 1] == i - 1;
-          if (!cont) { ch.push_back(start); ch.push_back(i); start = i; }
-        }
-      } else {
-        int end = n;   // current chain covers [i, end)
-        for (int i = n - 2; i >= -1; i--) {
-          const int r = i + 1;   // row just added
-          const bool cont = i >= 0 && end - i <= ILU_CHAIN_MAX && f.diag[i] + 1 < f.rowptr[i + 1] &&
-                            f.colidx[f.diag[i] + 1] == i + 1;
-          if (!cont) { ch.push_back(r); ch.push_back(end); end = r; }
-        }
-      }
-      const int nc = (int)ch.size() / 2;
-      for (int c = 0; c < nc; c++)
-        for (int i = ch[2 * c]; i < ch[2 * c + 1]; i++) chain_of[i] = c;
-      std::vector<int32_t> lev(nc, 0);
-      // chains are listed in dependency order (ascending rows for the lower
-      // solve, descending for the upper one), so one pass finds the levels
-      for (int c = 0; c < nc; c++) {
-        int d = 0;
-        for (int i = ch[2 * c]; i < ch[2 * c + 1]; i++) {
-          const int q0 = upper ? f.diag[i] + 1 : f.rowptr[i], q1 = upper ? f.rowptr[i + 1] : f.diag[i];
-          for (int q = q0; q < q1; q++) {
-            const int oc = chain_of[f.colidx[q]];
-            if (oc != c) d = std::max(d, lev[oc] + 1);
-          }
-        }
-        lev[c] = d;
-      }
-      nlev = 0;
-      for (int c = 0; c < nc; c++) nlev = std::max(nlev, lev[c] + 1);
-      std::vector<int32_t> cnt(nlev + 1, 0);
-      for (int c = 0; c < nc; c++) cnt[lev[c] + 1]++;
-      maxw = 0;
-      for (int k = 0; k < nlev; k++) maxw = std::max(maxw, cnt[k + 1]);
-      for (int k = 0; k < nlev; k++) cnt[k + 1] += cnt[k];
-      order.resize(nc);
-      for (int c = 0; c < nc; c++) order[cnt[lev[c]]++] = c;
-    };
-    chains(false, f.lchain, f.lchain_order, f.lchain_levels, f.lchain_maxw);
-    chains(true, f.uchain, f.uchain_order, f.uchain_levels, f.uchain_maxw);
+  // chains of the lower (ascending) and upper (descending) solves
+  for (int start = 0, i = 1; i <= n; i++) {
+    const bool cont = i < n && i - start < ILU_CHAIN_MAX && f.diag[i] > f.rowptr[i] && f.colidx[f.diag[i] - 1] == i - 1;
+    if (!cont) { f.lchain.push_back(start); f.lchain.push_back(i); start = i; }
+  }
+  for (int end = n, i = n - 2; i >= -1; i--) {   // the current chain covers [i + 1, end)
+    const bool cont = i >= 0 && end - i <= ILU_CHAIN_MAX && f.diag[i] + 1 < f.rowptr[i + 1] &&
+                      f.colidx[f.diag[i] + 1] == i + 1;
+    if (!cont) { f.uchain.push_back(i + 1); f.uchain.push_back(end); end = i + 1; }
   }
   // update lists: the upper blocks of every pivot row that row i's pattern holds
   {
@@ -371,6 +332,36 @@ std::string build_ilu_pattern(const Topology &t, int levels, int nblocks, IluPat
     }
   }
   return "";
+}
+
+std::vector<int32_t> chain_order(const IluPattern &f, bool upper, int &levels)
+{
+  const std::vector<int32_t> &ch = upper ? f.uchain : f.lchain;
+  const int nc = (int)ch.size() / 2;
+  std::vector<int32_t> chain_of(f.diag.size());
+  for (int c = 0; c < nc; c++)
+    for (int i = ch[2 * c]; i < ch[2 * c + 1]; i++) chain_of[i] = c;
+  // chains are listed in dependency order (ascending rows for the lower
+  // solve, descending for the upper one), so one pass finds the levels
+  std::vector<int32_t> lev(nc, 0);
+  levels = 0;
+  for (int c = 0; c < nc; c++) {
+    int d = 0;
+    for (int i = ch[2 * c]; i < ch[2 * c + 1]; i++) {
+      const int q0 = upper ? f.diag[i] + 1 : f.rowptr[i], q1 = upper ? f.rowptr[i + 1] : f.diag[i];
+      for (int q = q0; q < q1; q++) {
+        const int oc = chain_of[f.colidx[q]];
+        if (oc != c) d = std::max(d, lev[oc] + 1);
+      }
+    }
+    lev[c] = d;
+    levels = std::max(levels, d + 1);
+  }
+  std::vector<int32_t> cnt(levels + 1, 0), order(nc);
+  for (int c = 0; c < nc; c++) cnt[lev[c] + 1]++;
+  for (int k = 0; k < levels; k++) cnt[k + 1] += cnt[k];
+  for (int c = 0; c < nc; c++) order[cnt[lev[c]]++] = c;
+  return order;
 }
 
 }  // namespace cfdgpu

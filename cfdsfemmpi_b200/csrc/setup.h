@@ -77,22 +77,23 @@ struct IluPattern {
   // rows sorted by level of the lower DAG (factorisation and lower solve:
   // level(i) = 1 + max level of the strictly lower blocks' columns) and of
   // the upper DAG (upper solve), row order inside a level
-  std::vector<int32_t> lorder, uorder;
+  std::vector<int32_t> lorder, uorder, llev, ulev;   // llev, ulev: each row's level
   int nlev_l = 0, nlev_u = 0;
   int maxw_l = 0, maxw_u = 0;    // rows in the widest level of each DAG
   // chains of the triangular solves: maximal runs of consecutive rows in
   // which each row depends on its neighbour (row i on i-1 in the lower solve,
   // on i+1 in the upper solve), at most ILU_CHAIN_MAX rows.  A chain is solved
   // in order by one warp, so the dependency along it never goes through
-  // memory.  lchain/uchain: nchains x {first row, one past the last row};
-  // lchain_order/uchain_order: chain ids sorted by the level of the chain
-  // DAG (a chain's inputs lie in chains of lower levels).
-  std::vector<int32_t> lchain, uchain, lchain_order, uchain_order;
-  int lchain_levels = 0, uchain_levels = 0, lchain_maxw = 0, uchain_maxw = 0;
+  // memory.  lchain/uchain: nchains x {first row, one past the last row}.
+  std::vector<int32_t> lchain, uchain;
   int64_t nnzb() const { return (int64_t)colidx.size(); }
 };
 
 constexpr int ILU_CHAIN_MAX = 128;
+
+// Chain ids sorted by the level of the chain DAG (a chain's inputs lie in chains
+// of lower levels), and the number of levels.
+std::vector<int32_t> chain_order(const IluPattern &f, bool upper, int &levels);
 
 std::string build_ilu_pattern(const Topology &t, int levels, int nblocks, IluPattern &f);
 

@@ -28,17 +28,10 @@ void build_trsv_plan(const IluPattern &f, int nb, bool upper, TrsvPlan &p, bool 
   const int nc = (int)ch.size() / 2;
 
   // dependency level of every row (rows come to be solved in about this order)
-  std::vector<int32_t> lev(n, 0);
-  int levels = 0;
+  const std::vector<int32_t> &lev = upper ? f.ulev : f.llev;
+  const int levels = upper ? f.nlev_u : f.nlev_l;
   int64_t off = 0;
-  for (int s = 0; s < n; s++) {
-    const int i = upper ? n - 1 - s : s;
-    int d = 0;
-    for (int q = q0(i); q < q1(i); q++) d = std::max(d, lev[f.colidx[q]] + 1);
-    lev[i] = d;
-    levels = std::max(levels, d + 1);
-    off += q1(i) - q0(i);
-  }
+  for (int i = 0; i < n; i++) off += q1(i) - q0(i);
   const double at_once = (double)n / std::max(levels, 1);
 
   // segments: runs of consecutive chains (in solve order) each depending on
