@@ -35,8 +35,9 @@ def test_gradient_of_one_stage_matches_cpu_reference(where):
     in_s = np.concatenate([np.full(nd, 0.1), np.full(nd, 0.02)]).astype(np.float32)
     out_s = np.full(nd, 0.02, np.float32)
     net.set_scales(in_s, out_s)
-    us = [0.1 * rng.standard_normal(h.n) for _ in range(3)]
-    us[2].reshape(-1, nd)[first:first + STAGE] += 20.0 * rng.standard_normal((min(STAGE, mesh.nNode - first), nd))
+    us = [0.1 * rng.standard_normal(h.n) for _ in range(2)]
+    us.append(2 * us[1] - us[0])                                # targets of zero but for the stage's
+    us[2].reshape(-1, nd)[first:first + STAGE] += 2000.0 * rng.standard_normal((min(STAGE, mesh.nNode - first), nd))
     net.add_sample(*us, cond=0.3)
     p = net.get_params()
     off, _ = mpnn_ref.layout()
