@@ -12,16 +12,19 @@
 // order) and their streams get priorities by size (largest highest), so the
 // longest dependent kernel chains are not slowed by the small instances;
 // `concurrency` threads take part; `chunk` is the number of Arnoldi
-// steps per graph; `depth` the number of chunks a handle keeps enqueued
+// steps per graph (one outer step per graph in mixed precision, whatever it
+// says); `depth` the number of chunks a handle keeps enqueued
 // beyond the one whose state its host thread waits for (a sleeping thread
 // wakes up tens of microseconds after its event, so small instances need
 // more than one chunk in flight to keep their stream busy).  With all three
 // set to 0 the batch autotunes: the first batch steps try candidate
 // triples, one per step, scored by wall time per GMRES iteration of the
-// step, and the best is kept for the rest of the run.  No knob changes any
-// number an instance computes (kernels after GMRES convergence are no-ops and
-// every reduction has a fixed order), so each instance's results are bitwise
-// those of its own single-instance run.
+// step, and the best is kept for the rest of the run.  The number of instances
+// stepped at once also picks the forms of some kernels (those for a chip that is
+// shared do less work per sum).  No knob changes any number an instance computes
+// (kernels after GMRES convergence are no-ops and every reduction has a fixed
+// order, the same in all its forms), so each instance's results are bitwise those
+// of its own single-instance run.
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -83,7 +83,7 @@ struct cfdgpu_handle {
   double *bsr = nullptr;
   double *dinv = nullptr, *binv = nullptr;
   int m = 0;
-  int64_t ldv = 0;     // Krylov vector stride (multiple of 32 entries, zero padded)
+  int64_t ldv = 0;     // Krylov vector stride (multiple of 512 entries, zero padded)
   // mixed precision: FP64 flexible GMRES outer solve on the FP64 matrix, FP32
   // BiCGStab inner solves on an FP32 copy with an FP32 preconditioner
   bool mixed = false;

@@ -550,7 +550,7 @@ gmres_start(int64_t n, const VT *__restrict__ v0, GmresState *st, GmresArrays ga
 __device__ __forceinline__ int64_t hidx(int r, int c, int m) { return (int64_t)c * (m + 1) + r; }
 
 // Krylov vectors are stored with a leading dimension ldv that is a multiple
-// of 32 entries; entries n..ldv-1 stay zero, so every kernel below processes
+// of 512 entries; entries n..ldv-1 stay zero, so every kernel below processes
 // 16-byte chunks (Chunk<VT>::E entries) over nchunk = ldv / E.
 constexpr int ORTHO_THREADS = 256;
 constexpr int MDOT_KC = 8;          // basis vectors per CTA in the multi-dot
@@ -853,7 +853,7 @@ gmres_maxpy_norm(int64_t nchunk, VT *__restrict__ V, int64_t ldv, int j, GmresSt
     const int lp = threadIdx.x % CL, g = threadIdx.x / CL;
     const int64_t c0 = (int64_t)(blockIdx.x - 1) * SPAN;
     // the chunk of w this thread finishes, loaded early; nchunk is a multiple
-    // of 16 (ldv is one of 32 entries), the spans may reach past it
+    // of 128 (ldv is one of 512 entries), the spans may reach past it
     const int64_t pfin = c0 + threadIdx.x;
     const bool fin = threadIdx.x < SPAN && pfin < nchunk;
     double wfin[E];

@@ -429,7 +429,8 @@ int cfdgpu_batch_size(cfdgpu_batch *b);
 /* instance i's handle (get/set solution, history, timers...); owned by the batch */
 cfdgpu_handle *cfdgpu_batch_handle(cfdgpu_batch *b, int i);
 /* concurrency: host threads stepping instances at once; chunk: Arnoldi steps
- * per CUDA graph (1..64); depth: chunks each instance keeps enqueued beyond
+ * per CUDA graph (1..64; a mixed-precision solve has one outer step per graph
+ * whatever it says); depth: chunks each instance keeps enqueued beyond
  * the one whose state its thread waits for (1..8).  (0, 0, 0) = autotune:
  * the next batch steps each try one candidate, scored by wall time per GMRES
  * iteration, and the best is kept.  Results do not depend on any of them. */
