@@ -368,7 +368,8 @@ int cfdgpu_mpnn_set_condition(cfdgpu_mpnn *m, double cond);
  * meshes.  The other mesh must have the same dofs per node and dimension and
  * at most as many nodes as the network's own; predictions always serve the
  * network's own handle (copy trained weights into a network per instance
- * with cfdgpu_mpnn_get_params / cfdgpu_mpnn_set_params). */
+ * with cfdgpu_mpnn_get_params / cfdgpu_mpnn_set_params).  The network keeps
+ * the other handle's graph: destroy it, as its own handle, after the network. */
 int cfdgpu_mpnn_add_sample_on(cfdgpu_mpnn *m, cfdgpu_handle *h, double cond, const double *u_nm1, const double *u_n,
                               const double *u_np1);
 int cfdgpu_mpnn_num_samples(cfdgpu_mpnn *m);
